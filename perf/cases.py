@@ -30,7 +30,7 @@ def listed() -> list:
     return [
         # one query of a few sample points on a small cladded crystal: an interactive caller; launches and host work count
         dict(name="query", kind="solve", proposal="walks", rings=6, levels=5, lambdas=1, reflect=False, cladding=True,
-             samples=5, rays=10_000, max_rays=5_000),
+             samples=5, rays=10_000, max_rays=10_000),
         # the whole small disc, one wavelength, adaptive to 0.5 % error: the everyday monochromatic solve
         dict(name="disc_mono", kind="solve", proposal="walks", rings=13, levels=10, lambdas=1, reflect=False,
              cladding=False, samples=0, rays=100_000, max_rays=1_000_000),
