@@ -770,6 +770,41 @@ __device__ __forceinline__ uint32_t upperBound(const uint32_t* a, uint32_t n, ui
     return lo;
 }
 
+// The map entries of a warp's next rays, r for each lane (rays of consecutive
+// lanes do not decrease; entry b holds the rays [off[b], off[b + 1])).  b0: an
+// entry at or before that of the first ray, end: past the last entry of the
+// item.  The warp reads 32 offsets `1 << shift` entries apart with one load
+// and every lane finds its interval among them by shuffles, then its entry
+// inside the interval; shift (entryShift) makes the 32 intervals span about
+// twice the entries that 32 rays take, so that a lane beyond them (it searches
+// the rest) is rare.  Each lane's own binary search over the item's entries
+// took 7 (one ray per entry and more) to 13 (5 entries per ray) dependent
+// loads and 9 instructions for each.
+__device__ __forceinline__ uint32_t warpEntries(const uint32_t* off, uint32_t b0, uint32_t end, uint32_t shift,
+                                                uint32_t r) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t v = __ldg(off + min(b0 + ((lane + 1u) << shift), end));
+    uint32_t n = 0;  // offsets among the 32 that do not exceed r
+#pragma unroll
+    for (uint32_t step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, v, n + step - 1u) <= r) n += step;
+    const bool beyond = __shfl_sync(0xffffffffu, v, 31) <= r;
+    uint32_t b = b0 + (n << shift);
+    if (beyond) {
+        b = min(b0 + (32u << shift), end);
+        b += upperBound(off + b, end - b, r);
+        return b - 1u;
+    }
+    for (uint32_t step = (1u << shift) >> 1; step > 0; step >>= 1)
+        if (__ldg(off + min(b + step, end)) <= r) b += step;
+    return b;
+}
+
+// log2 of the entries between warpEntries' offsets for `rays` rays in `entries` entries.
+__device__ __forceinline__ uint32_t entryShift(uint32_t entries, uint32_t rays) {
+    return entries <= rays ? 0u : 31u - uint32_t(__clz(int(2u * entries / rays)));
+}
+
 // Start state of ray r of sample `sample`, drawn in reflection slice j and
 // prism p with probability qf / Q (qf: the map's integer weight q of the
 // entry, or the local proposal's mixture weight): Philox4x32-10 counter (r,
@@ -981,7 +1016,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
 #define HASE_SPEC (POOL ? (const float2*)iv.spec : L.spec)
         const double Cm = POOL ? double(iv.C) : double(L.C);
         const MeshView& m = POOL ? sInst[threadIdx.x >> 5].m : L.m;
-        const GlobalLoader load{m.walk};
         const uint32_t r0 = k * L.itemRays;
         const uint32_t r1 = min(r0 + L.itemRays, L.M);
         const uint32_t* off = L.offsets + oBase;
@@ -1006,6 +1040,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
         double sum = 0.0, sum2 = 0.0;
         uint32_t dropped = 0, crossings = 0;
         uint32_t fetch = r0;
+        uint32_t bNext = pb;  // an entry at or before the next ray's
+        const uint32_t shift = LOCAL ? 0u : entryShift(count, r1 - r0);
         bool active = false;
         Ray ray;
         float wf = 0.0f;
@@ -1016,6 +1052,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
             if (fetch >= r1 && nIdle == 32) break;
             if (fetch < r1 && (nIdle >= REFILL || nIdle == 32)) {
                 const uint32_t r = fetch + __popc(idle & laneLt);
+                uint32_t entry = 0;
+                if constexpr (!LOCAL) {
+                    entry = warpEntries(off, bNext, pb + count - 1u, shift, min(r, r1 - 1u));
+                    bNext = __shfl_sync(0xffffffffu, entry, 31 - __clz(int(idle)));
+                }
                 if (!active && r < r1) {
                     uint32_t j = 0, p = 0;
                     float qf = 1.0f;
@@ -1026,7 +1067,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
                                          qf, bl);
                         if (LOG) bsel = bl;
                     } else {
-                        const uint32_t b = pb + upperBound(off + pb, count, r) - 1u;
+                        const uint32_t b = entry;
                         if (LOG) bsel = b;
                         // reflection slice by subtraction (at most 4)
                         p = b;
@@ -1046,9 +1087,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
                 fetch += uint32_t(nIdle);
             }
             if (active) {
-                const int st = stepRay<COLS, WALK>(m, S.x, S.y, ray, load);
+                const int st = stepRay<COLS, WALK>(m, S.x, S.y, ray);
                 if (st != kContinue) {
-                    crossings += uint32_t(ray.steps) + 1u;
+                    crossings += uint32_t(raySteps(ray)) + 1u;
                     if (st == kDone) {
                         finishReflections(m, ray);
                         // the ray's gain in FP32 (FP64 only where exp(G)
@@ -1278,10 +1319,9 @@ __global__ void traceKernel(TraceLaunch L) {
     Ray r;
     const float D2 = initRay(r, L.tri[i], int(L.level[i]), L.start[3 * i] - S.x, L.start[3 * i + 1] - S.y,
                              L.start[3 * i + 2] - zImgOffset, kImg, j, L.A, L.B, m);
-    GlobalLoader load{m.walk};
     int st;
     do {
-        st = stepRay(m, S.x, S.y, r, load);
+        st = stepRay(m, S.x, S.y, r);
     } while (st == kContinue);
     if (st == kDone) finishReflections(m, r);
     L.lnGain[i] = r.G;
@@ -1854,7 +1894,7 @@ void invariantDivisor(uint32_t d, uint32_t& mul, uint32_t& shift) {
 
 struct HostTables {
     std::vector<int4> verts;
-    std::vector<float4> tri, walk, geo;
+    std::vector<float4> tri, walk, win, geo;
     std::vector<float2> centroid, points;
 };
 
@@ -1932,6 +1972,23 @@ hase_status buildHostTables(const hase_mesh_desc* d, HostTables& h, double& exte
             std::memcpy(&nb, r + 9 + e, sizeof(nb));
             if (nb < 0) r[kNx[e]] = r[kNy[e]] = nan;
         }
+    }
+    // the ray walk's windows: the same edges in the slots e0 e1 e2 e0
+    h.win.resize(4 * size_t(T));
+    for (uint32_t t = 0; t < T; ++t) {
+        const float* r = &h.walk[3 * size_t(t)].x;
+        for (int e = 0; e < 3; ++e) {
+            int32_t nb;
+            std::memcpy(&nb, r + 9 + e, sizeof(nb));
+            float4& w = h.win[4 * size_t(t) + e];
+            w = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+            if (nb < 0) continue;
+            static const int kAt[3] = {0, 3, 6};
+            const uint32_t code = (uint32_t(nb) & ~3u) | windowSlot(uint32_t(nb) & 3u);
+            w = make_float4(r[kAt[e]], r[kAt[e] + 1], r[kAt[e] + 2], 0.0f);
+            std::memcpy(&w.w, &code, sizeof(code));
+        }
+        h.win[4 * size_t(t) + 3] = h.win[4 * size_t(t)];
     }
     return HASE_OK;
 }
@@ -2176,7 +2233,7 @@ struct hase_context {
     std::vector<double> betaCells, sigmaA, sigmaE;
     bool hasReflect = false;
     float tirCos2[2] = {-1.0f, -1.0f};
-    DevBuf<float4> tri, walk, geo;
+    DevBuf<float4> tri, walk, win, geo;
     DevBuf<int4> verts;
     DevBuf<uint16_t> lineOrder[2];  // importance line order per sample level: 1 and 5 reflection slices
     // local proposal (hase_context_set_local_proposal): per point the K
@@ -2233,6 +2290,7 @@ struct hase_context {
         invariantDivisor(Np, v.divNpm, v.divNps);
         v.tri = tri.p;
         v.walk = walk.p;
+        v.win = win.p;
         v.geo = geo.p;
         v.verts = verts.p;
         v.centroid = centroid.p;
@@ -2667,6 +2725,7 @@ hase_status hase_context_create(const hase_mesh_desc* d, const hase_spectrum_des
     };
     if ((st = up(c->tri, ht.tri)) != HASE_OK) return cleanup(st);
     if ((st = up(c->walk, ht.walk)) != HASE_OK) return cleanup(st);
+    if ((st = up(c->win, ht.win)) != HASE_OK) return cleanup(st);
     if ((st = up(c->geo, ht.geo)) != HASE_OK) return cleanup(st);
     if ((st = up(c->verts, ht.verts)) != HASE_OK) return cleanup(st);
     if (uint64_t(5) * c->layers < 65536) {  // importance line order (16-bit line indices)

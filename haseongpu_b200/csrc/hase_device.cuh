@@ -69,7 +69,8 @@ __device__ __forceinline__ float unit24(uint32_t k24) { return (float(k24) + 0.5
 //   g0 = (ax, ay, bx-ax, by-ay), g1 = (cx-ax, cy-ay, area, 0); centroid separate.
 struct MeshView {
     const float4* tri;       // [T][3]
-    const float4* walk;      // [T][3]: tri with NaN normals on mesh-boundary edges (the walks' records)
+    const float4* walk;      // [T][3]: tri with NaN normals on mesh-boundary edges (the importance walks' records)
+    const float4* win;       // [T][4]: the ray walk's edge windows (kWindowSlot)
     const float4* geo;       // [T][2]
     const int4* verts;       // [T] point ids of the triangle's vertices (w unused)
     const float2* centroid;  // [T]
@@ -91,6 +92,18 @@ struct MeshView {
     float tolEnd;            // |s| below which the target is reached
     float tirCos2[2];        // total internal reflection when uz^2 <= tirCos2[surface]
 };
+
+// The ray walk's edge windows.  An edge is one float4 (nx, ny, c, code), a
+// triangle holds its edges in the four slots e0 e1 e2 e0, and a window is the
+// pair of slots a ray that entered through the third edge can leave by:
+// entered through e0: slots 1, 2; e1: slots 2, 3; e2: slots 0, 1.  code is the
+// window on the other side, 4 neighbour + its first slot, so that one index,
+// loaded with the edge, is the next triangle, its records' address and the
+// edge that is left out.  The three-edge records cost a third edge test and a
+// third 16-byte load per triangle for an edge that never is the exit.
+// A mesh-boundary edge is (0, 0, 1, 0): its exit parameter is negative whatever
+// the ray, so it is never chosen, and its code is a valid index.
+__host__ __device__ __forceinline__ uint32_t windowSlot(uint32_t entryEdge) { return entryEdge == 2 ? 0u : entryEdge + 1u; }
 
 // Layer of prism index p < 2^31 (p = t + layer T): an exact multiply-shift
 // instead of a 32-bit division by the runtime T.
@@ -129,11 +142,11 @@ __device__ __forceinline__ float reflectFactor(const MeshView& m, uint32_t t, in
 // image point, +T or -T (it flips at every reflection), so no division, modulo
 // or multiplication is needed per crossing.
 struct Ray {
-    uint32_t t;     // triangle
+    uint32_t w;     // edge window: 4 triangle + first slot (MeshView::win)
     int row;        // physical layer of the current unfolded layer, times T
     int rstep;      // +T / -T
     int reflLeft;   // reflections the slice still implies
-    int steps;
+    int steps;      // triangles left minus the first zl: with the current zl, the crossings so far (raySteps)
     float s;        // remaining distance to the image point
     float G;        // accumulated ln(gain) for the pair (A, B), including reflection factors
     float A, B;     // g = beta*A - B: the walk's reference pair
@@ -148,6 +161,9 @@ struct Ray {
     float hOverUz;
     float zl;
 };
+
+// Crossings so far: triangles left plus level planes and reflections.
+__device__ __forceinline__ int raySteps(const Ray& r) { return r.steps + int(r.zl); }
 
 enum StepResult { kContinue = 0, kDone = 1, kDropped = 2 };
 
@@ -173,10 +189,8 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     const float D2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const float D = sqrtf(D2);
     const float inv = 1.0f / D;
-    r.t = t;
     r.row = layer * int(m.T);
     r.reflLeft = expectedReflections(slice);
-    r.steps = 0;
     r.s = D;
     r.G = 0.0f;
     r.Jb = 0.0f;
@@ -188,10 +202,18 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     // moving toward the image: down (layer step -1) when uz > 0, up (+1) otherwise
     const float hu = __fdividef(h, r.uz);
     r.hOverUz = r.uz > 0.0f ? -hu : hu;
-    r.zl = r.uz > 0.0f ? float(kImg - layer) : float(layer + 1 - kImg);
+    const int zl0 = r.uz > 0.0f ? kImg - layer : layer + 1 - kImg;
+    r.zl = float(zl0);
+    r.steps = -zl0;
     r.rstep = r.uz > 0.0f ? -int(m.T) : int(m.T);
     r.A = A;
     r.B = B;
+    // the first window leaves out an edge the ray does not move out through
+    // (one of the three always is; a boundary edge's zero normal counts too)
+    const float2* e = reinterpret_cast<const float2*>(m.win + 4 * size_t(t));
+    const float2 e0 = __ldg(e), e1 = __ldg(e + 2);
+    const bool out0 = -fmaf(e0.x, r.ux, e0.y * r.uy) > 0.0f, out1 = -fmaf(e1.x, r.ux, e1.y * r.uy) > 0.0f;
+    r.w = 4 * t + (!out0 ? 1u : (!out1 ? 2u : 0u));
     return D2;
 }
 
@@ -236,95 +258,132 @@ __device__ __forceinline__ double rayMeanGain(const Ray& r, const float2* spec, 
     return e * double(sum) / double(nL);
 }
 
-// One triangle column: the edge exit of the current triangle (edge exits are
-// compared as fractions num/den by cross multiplication; one approximate
-// division gives the chosen exit parameter), then every level plane crossed
-// before it.
-// Walks up to K triangle columns per call.  Once a column's exit edge is
-// known, the next triangle's walk record is loaded (into the registers the
-// current record no longer needs) while the current column's level planes are
-// worked through, so its latency is hidden behind them.
-// The walk is bound by instruction issue, so the level-plane loop is kept
-// short: the step bound is checked once per call (the loop itself ends
-// within 3 x layers crossings: every physical layer step reaches a surface and
-// at most two reflections are allowed), and kWalkTable walks the table of g = beta A
-// - B (m.gTab) instead of evaluating it at every crossing (WalkMode).
-template <int K = 1, int WALK = kWalkBeta, typename Loader>
-__device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ray& r, Loader&& load) {
+// Reciprocal with the hardware approximation (1 ulp; subnormal inputs give inf).
+__device__ __forceinline__ float rcpApprox(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Exit parameter s = e / d of one window edge for a ray along -u to the sample:
+// d the speed out through the edge, e the sample's signed distance from its
+// line.  Negative unless the ray moves out: e takes d's sign bit where that is
+// set.  (In through an edge, d < 0, the sample lies on its inner side, e < 0,
+// up to the rounding of a ray that starts on the edge; without the sign such a
+// ray could step back and forth around a vertex.  The 1e-30 gives a ray along
+// the edge, d = 0, the same sign.)
+__device__ __forceinline__ float edgeExit(const float4& a, float ux, float uy, float Sx, float Sy) {
+    const float d = fmaf(-a.x, ux, fmaf(-a.y, uy, -1e-30f));
+    const float e = fmaf(a.x, Sx, fmaf(a.y, Sy, -a.z));
+    const float es = __uint_as_float(__float_as_uint(e) | (__float_as_uint(d) & 0x80000000u));
+    return es * rcpApprox(fabsf(d));
+}
+
+// A ray that stepped past a physical bottom or top surface in triangle t:
+// back into its layer, reflected (false: more reflections than the slice implies).
+__device__ __forceinline__ bool reflectRay(const MeshView& m, Ray& r, uint32_t t) {
+    if (r.reflLeft <= 0) return false;
+    r.G += __logf(reflectFactor(m, t, r.row < 0 ? 0 : 1, r.uz));
+    --r.reflLeft;
+    r.row -= r.rstep;
+    r.rstep = -r.rstep;
+    return true;
+}
+
+// Walks up to K triangle columns per call.  Per column: the exit is the later
+// crossing of the window's two edges, then the level planes before it.  Once the exit edge is known the next window's records are
+// loaded, so that their latency is hidden behind the column's planes.
+// The walk is bound by instruction issue and, within it, by the half-rate ALU
+// pipe (compares, selects, min/max, integers), so a column is straight-line
+// code with as few of those as it can do with:
+// - an edge the ray moves in through gets a negative exit parameter, which
+//   loses against any exit (edgeExit: two reciprocals on the idle
+//   special-function pipe in place of sign tests, a cross multiplication and
+//   their selects);
+// - no lower clamp: what is not above tolEnd, NaN included, is the target's
+//   column, whose end is 0;
+// - the segment to the first plane or the exit, and the segment after one
+//   plane (of no length where none is crossed: it adds exactly 0), are always
+//   computed; only lanes with a second plane in the column enter a loop.  A
+//   loop over the planes ran for the whole warp as often as its worst lane
+//   needed.
+// Crossings are counted by the columns and zl, the step bound is checked once
+// per call, and kWalkTable walks the table of g = beta A - B (m.gTab).
+// Boundary edges are never exits: the 2-D mesh is convex and the target lies
+// in it, so only rounding could route a ray across one.
+template <int K = 1, int WALK = kWalkBeta>
+__device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ray& r) {
     const float* gcol = WALK == kWalkTable ? m.gTab : m.gainBeta;
-    float4 a, b, c;
-    load(r.t, a, b, c);
+    const float4* win = m.win;
+    float4 a = __ldg(win + r.w), b = __ldg(win + r.w + 1);
     // beta (kWalkTable: g) of the current prism, issued with the record so
     // that its latency overlaps the edge tests
-    float gb = __ldg(gcol + r.row + r.t);
+    float gb = __ldg(gcol + r.row + (r.w >> 2));
 #pragma unroll 1
     for (int k = 0; k < K; ++k) {
-        float bn = -1.0f, bd = 0.0f;  // best fraction so far (-1/0 = -inf)
-        int bw = -1;
-        const auto edge = [&](float nx, float ny, float cc, int nbw) {
-            const float dd = -fmaf(nx, r.ux, ny * r.uy);       // > 0: moving out through the edge
-            const float nm = fmaf(nx, Sx, fmaf(ny, Sy, -cc));  // signed distance of the sample from the edge line
-            // Boundary edges are never exits: the 2-D mesh is convex and the
-            // target lies in it, so only rounding could route a ray across one.
-            // The walk records (MeshView::walk) give them NaN normals, so
-            // their dd > 0 test fails.  The entry edge needs no test either:
-            // the two triangles of an edge store exactly negated normals (both
-            // are computed in FP64 from the same two points and rounded), so
-            // the entry edge's dd is exactly minus the dd > 0 it was chosen
-            // with in the previous triangle.
-            const bool ok = dd > 0.0f;
-            if (ok && nm * bd > bn * dd) {
-                bn = nm;
-                bd = dd;
-                bw = nbw;
+        const uint32_t t = r.w >> 2;
+        const float q1 = edgeExit(a, r.ux, r.uy, Sx, Sy), q2 = edgeExit(b, r.ux, r.uy, Sx, Sy);
+        const float qm = fmaxf(q1, q2);
+        const uint32_t code = __float_as_uint(q2 == qm ? b.w : a.w);
+        a = __ldg(win + code);
+        b = __ldg(win + code + 1);
+        const float sEdge = fminf(qm, r.s);
+        const float cut = fmaxf(sEdge, m.tolEnd);
+        const bool last = !(sEdge > m.tolEnd);  // the target's column: its planes above tolEnd, then the rest of the path
+        const float sEnd = last ? 0.0f : sEdge;
+        float sz = r.zl * r.hOverUz;
+        bool plane = sz > cut;
+        float next = plane ? sz : sEnd;
+        addSegment<WALK>(r, gb, r.s - next, m.cladAbs);
+        r.s = next;
+        if (plane) {
+            r.row += r.rstep;
+            r.zl += 1.0f;
+        }
+        if (uint32_t(r.row) >= m.P) {
+            if (!reflectRay(m, r, t)) {
+                r.steps += k;
+                return kDropped;
             }
-        };
-        edge(a.x, a.y, a.z, __float_as_int(c.y));
-        edge(a.w, b.x, b.y, __float_as_int(c.z));
-        edge(b.z, b.w, c.x, __float_as_int(c.w));
-        // clamped at 0: the comparison sz < sEdge below is reached only with
-        // sz > tolEnd >= 0, where the clamp does not change it
-        const float sEdge = fmaxf(fminf(__fdividef(bn, bd), r.s), 0.0f);
-        if (K > 1 && k + 1 < K && bw >= 0) load(uint32_t(bw) >> 2, a, b, c);
-        // Level planes crossed before the edge exit: the triangle, and with it
-        // sEdge, stays the same, so they cost no edge test.
-        while (true) {
-            const float sz = fminf(r.zl * r.hOverUz, r.s);
-            const float next = fmaxf(sEdge, sz);
-            if (next <= m.tolEnd) {
-                addSegment<WALK>(r, gb, r.s, m.cladAbs);
-                r.s = 0.0f;
-                return kDone;
+        }
+        gb = __ldg(gcol + r.row + t);
+        sz = r.zl * r.hOverUz;
+        plane = plane && sz > cut;
+        next = plane ? sz : sEnd;
+        addSegment<WALK>(r, gb, r.s - next, m.cladAbs);
+        r.s = next;
+        while (plane) {
+            r.row += r.rstep;
+            r.zl += 1.0f;
+            if (uint32_t(r.row) >= m.P && !reflectRay(m, r, t)) {
+                r.steps += k;
+                return kDropped;
             }
+            gb = __ldg(gcol + r.row + t);
+            sz = r.zl * r.hOverUz;
+            plane = sz > cut;
+            next = plane ? sz : sEnd;
             addSegment<WALK>(r, gb, r.s - next, m.cladAbs);
             r.s = next;
-            ++r.steps;
-            if (sz < sEdge) break;
-            const int cand = r.row + r.rstep;
-            if (uint32_t(cand) >= m.P) {  // a physical bottom/top surface: reflect
-                if (r.reflLeft <= 0) return kDropped;
-                r.G += __logf(reflectFactor(m, r.t, cand < 0 ? 0 : 1, r.uz));
-                --r.reflLeft;
-                r.rstep = -r.rstep;
-            } else {
-                r.row = cand;
-            }
-            r.zl += 1.0f;
-            gb = __ldg(gcol + r.row + r.t);
         }
-        r.t = uint32_t(bw) >> 2;
-        if (K > 1 && k + 1 < K) gb = __ldg(gcol + r.row + r.t);
+        if (last) {
+            r.steps += k;
+            return kDone;
+        }
+        r.w = code;
+        gb = __ldg(gcol + r.row + (code >> 2));
     }
+    r.steps += K;
     // the step bound, once per call: a call walks at most K columns of at most
     // 1 + 3 x layers segments each
-    return r.steps >= kMaxSteps ? kDropped : kContinue;
+    return raySteps(r) >= kMaxSteps ? kDropped : kContinue;
 }
 
 // After kDone: a reflection the slice implies but which happens at the target
 // itself (a sample on the reflecting surface) is applied in the final triangle.
 __device__ __forceinline__ void finishReflections(const MeshView& m, Ray& r) {
     if (r.reflLeft > 0) {
-        r.G += __logf(reflectFactor(m, r.t, r.row + r.rstep < 0 ? 0 : 1, r.uz));
+        r.G += __logf(reflectFactor(m, r.w >> 2, r.row + r.rstep < 0 ? 0 : 1, r.uz));
         r.reflLeft = 0;
     }
 }

@@ -1,0 +1,84 @@
+"""The ray kernel's search of the ray map and the grouping of the importance walks, at the sizes where they can go
+wrong: entries per ray below and above one, weights that leave lanes beyond the searched interval, ray counts around
+a warp and a work item; line counts around the teams' sizes, several levels of a point in one team."""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import legacy_mesh, legacy_spectrum
+
+pytestmark = pytest.mark.gpu
+
+
+def _weights(kind, n, rng):
+    if kind == "uniform":
+        return np.ones(n)
+    if kind == "one_heavy":  # almost every ray in one entry, the rest of the entries share a few
+        w = np.full(n, 1e-7)
+        w[n // 3] = 1.0
+        return w
+    if kind == "clusters":  # runs of empty entries between dense ones
+        w = np.zeros(n)
+        w[:: max(1, n // 37)] = 1.0
+        w[5:9] = 1e-3
+        return w
+    return rng.random(n) ** 12  # "spiky"
+
+
+@pytest.mark.parametrize("kind", ["uniform", "one_heavy", "clusters", "spiky"])
+@pytest.mark.parametrize("rays", [1, 31, 33, 1000, 70_000])
+def test_rays_follow_the_map(oracle, native, kind, rays):
+    """Every ray starts in its map entry: the estimate from the caller's weights equals the oracle's replay of the same
+    rays (the parity level of the replays, 1e-4)."""
+    import torch
+
+    from haseongpu_b200 import DeviceMesh
+
+    mesh = legacy_mesh("cylindrical")
+    sa, se = legacy_spectrum("cylindrical")
+    w = np.where(mesh.betaVolume > 0, _weights(kind, mesh.numberOfPrisms, np.random.default_rng(1)), 0.0).astype(np.float32)
+    sample = 2050
+    with DeviceMesh(mesh, sa, se) as ctx:
+        d_w, d_out = torch.from_numpy(w).cuda(), torch.zeros(4, dtype=torch.float64, device="cuda")
+        native.check(native.lib().hase_estimate_sample_noalloc(ctx.handle, sample, C.c_void_p(d_w.data_ptr()), rays, 9,
+                                                               0, 1, C.c_void_p(d_out.data_ptr())))
+        got = d_out.cpu().numpy()
+    ref = oracle.phi_ase(mesh, (sa, se), minRays=rays, seed=9, minSample=sample, maxSample=sample, weights=w[None])
+    assert got[2] == rays and got[3] == 0
+    np.testing.assert_allclose(got[0], float(ref["phiAse"][0]), rtol=1e-4)
+
+
+@pytest.mark.parametrize("levels,reflections", [(2, False), (4, False), (6, False), (9, True), (3, True), (14, True)])
+def test_grouped_levels_give_the_single_rows(oracle, levels, reflections):
+    """A range over every level of every point walks a point's levels together (1 to 13 layers, 2 to 14 levels, 1 or 5
+    slices: 2 to 910 lines); the same rows one by one give the same bits, and the oracle's weights to the replays' 1e-5
+    for 99.9 % (5e-4 for all: a line that grazes an edge)."""
+    from haseongpu_b200 import DeviceMesh, PrismMesh
+    from haseongpu_b200.mesh import delaunay_triangles, disc_points, gaussian_pump_beta
+
+    rng = np.random.default_rng(levels)
+    pts = disc_points(0.8, 4, rng)
+    tri = delaunay_triangles(pts)
+    T = tri.shape[0]
+    mesh = PrismMesh(points=pts, triangles=tri, numberOfLevels=levels, thickness=0.5 / levels,
+                     betaVolume=gaussian_pump_beta(pts, tri, levels, 0.5 / levels), nTot=1.38e20, crystalTFluo=1e-3,
+                     reflectivities=np.tile([0.3, 0.9], (T, 1)), refractiveIndices=[1.83, 1.0, 1.5, 1.0])
+    spectrum = ([1.1e-21], [2.2e-20])
+    S = mesh.numberOfSamples
+    with DeviceMesh(mesh, *spectrum) as ctx:
+        every = ctx.importance_weights(0, S, reflections)
+        picks = [0, pts.shape[0] - 1, S // 2, S - 1]
+        for s in picks:
+            np.testing.assert_array_equal(ctx.importance_weights(s, 1, reflections)[0], every[s])
+        part = ctx.importance_weights(3, S - 7, reflections)
+        np.testing.assert_array_equal(part, every[3:S - 4])
+    for s in picks:
+        ref = np.asarray(oracle.importance(mesh, spectrum, s, slices=5 if reflections else 1), float).ravel()
+        ref = ref / ref.max()
+        big = ref > 1e-6
+        rel = np.abs(every[s][big] / ref[big] - 1.0)
+        assert np.quantile(rel, 0.999) < 1e-5 and rel.max() < 5e-4
