@@ -69,7 +69,7 @@ def autotune(ctx, *, firstSample: int, samples: int, rays: int, useReflections: 
             if best is None or t < best[2]:
                 best = (v, rpt, t)
     imp = []
-    for layers in (0, 2, 4, 8):  # 0: the line-team kernel
+    for layers in (0,):  # the line-team kernel: the one importance kernel there is
         t = min(ctx.calc_phi_ase(minRays=1, maxRays=1, useReflections=useReflections, monochromatic=monochromatic,
                                  nearFieldSampling=nearFieldSampling, rngSeed=3, minSample=firstSample,
                                  maxSample=firstSample + samples - 1, importanceLayers=layers).importanceMilliseconds

@@ -2,9 +2,9 @@
 // importance-sampled phi-ASE method and the C ABI around them.
 //
 // Per batch of sample points (prism mesh, FP32 geometry, FP64 sums):
-//   (a1) importanceKernel  one thread per (sample, reflection slice, prism):
-//        straight-line walk from the prism centre to the (image) sample point,
-//        ln w = ln(beta V / d^2) + Int g dl.
+//   (a1) importanceTeamKernel  a team of lanes per (sample point, triangle):
+//        straight-line walks from the prism centres to the (image) sample
+//        points, ln w = ln(beta V / d^2) + Int g dl.
 //   (a2) mapKernel         one CTA per sample: w = exp(ln w - max), integer
 //        quantisation q = ceil(w 2^24 / max w), warp-shuffle scans of q over
 //        one contiguous segment per warp and the systematic-sampling ray offsets
@@ -100,13 +100,24 @@ __device__ __forceinline__ T warpInclusiveScan(T v) {
     return v;
 }
 
+// Multiplier and shift with floor(n / d) = (n * mul) >> shift for every
+// n < 2^31 and 1 <= d < 2^32 (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", PLDI 1994, theorem 4.2 with N = 31):
+// l = ceil(log2 d), mul = ceil(2^(31 + l) / d) (< 2^32), shift = 31 + l.
+void invariantDivisor(uint32_t d, uint32_t& mul, uint32_t& shift) {
+    uint32_t l = 0;
+    while ((uint64_t(1) << l) < d) ++l;
+    shift = 31 + l;
+    mul = uint32_t(((uint64_t(1) << shift) + d - 1) / d);
+}
+
 // --------------------------------------------------------- (a1) weights ----
 struct ImportanceLaunch {
     MeshView m;
-    uint32_t firstSample, slices, nW;
-    float A, B;   // spectrally averaged gain coefficients
+    uint32_t firstSample, rows, slices, nW;
+    const float2* line;  // [T][phases layers]: lineTableKernel
     float* lnw;   // [rows][nW]
-    const uint32_t* rowList;  // rows to compute (blockIdx.y indexes it), or null: rows 0 .. gridDim.y - 1
+    const uint32_t* rowList;  // rows to compute (blockIdx.y indexes it), or null: rows 0 .. rows - 1
     const uint8_t* rowFlag;   // batched media: only rows with rowFlag[flagBase + row] set are computed (or null)
     uint32_t flagBase;
     unsigned long long* crossings;  // counting launches only: total walk crossings
@@ -114,302 +125,218 @@ struct ImportanceLaunch {
     // row then holds slices x layers x K entries (j (layers K) + l K + k)
     const uint32_t* cand;
     uint32_t K;
+    uint32_t divLm, divLs;  // floor(x / layers) = (x * divLm) >> divLs
 };
 
-// One thread per (sample, reflection slice, triangle, group of G layers): the
-// straight lines from the centres of the G prisms (t, l) to the (image)
-// sample point all project onto the same 2-D segment, centroid -> sample
-// point, so they cross the same triangles at the same 2-D distances sigma.
-// The thread walks that 2-D segment once (edge tests shared by the G lines)
-// and, per line, the level planes and top/bottom reflections inside each
-// triangle: plane k of line l lies at sigma = D2 (k - kImg) / (l + 1/2 - kImg).
-// ln w = ln(beta V / d^2) + Int g dl, Int g dl = (D3 / D2) Int g dsigma.
-// TAB: g of every prism is read from m.gTab (built for L.A, L.B) instead of
-// being evaluated from beta at every crossing.
-template <int G, bool TAB = false>
-__global__ void __launch_bounds__(256) importanceKernel(ImportanceLaunch L) {
-    const MeshView& m = L.m;
-    const float* gcol = TAB ? m.gTab : m.gainBeta;
-    const uint32_t groups = (m.layers + G - 1) / G;
-    const uint32_t perSlice = groups * m.T;
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= L.slices * perSlice) return;
-    const uint32_t row = L.rowList ? L.rowList[blockIdx.y] : blockIdx.y;
-    if (L.rowFlag && !L.rowFlag[L.flagBase + row]) return;
-    const uint32_t j = idx / perSlice;
-    const uint32_t rem = idx - j * perSlice;
-    const uint32_t grp = rem / m.T, t = rem - grp * m.T;
-    const int l0 = int(grp * G);
-    const uint32_t sample = L.firstSample + row;
-    const float2 S = __ldg(m.points + sample % m.Np);
-    const int ls = int(sample / m.Np);
-    const int kImg = imageLevel(ls, int(m.layers), j);
-    const float2 c = __ldg(m.centroid + t);
-    const float area = __ldg(&m.geo[2 * t + 1].z);
-    const float dx = c.x - S.x, dy = c.y - S.y;
-    const float D2 = sqrtf(fmaf(dx, dx, dy * dy));
-    const float inv2 = 1.0f / D2;
-    const float ux = dx * inv2, uy = dy * inv2;
-    float* out = L.lnw + size_t(row) * L.nW + size_t(j) * m.P + t;
-
-    float J[G], lnR[G], invc[G];
-    // the line's next level plane lies at s = kf * invc: kf is the plane's
-    // level offset from the image level (an exact small-integer float) and
-    // invc the distance per level, both times the line's layer step toward the
-    // image level, so that kf grows by 1 per plane
-    float kf[G];
-    // lrow: the line's physical layer x T; rstep: the row offset of the next
-    // physical layer toward the image level (+-T, flipped at a reflection)
-    int lrow[G], rstep[G], left[G];
-    bool ok[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const int l = l0 + g;
-        ok[g] = l < int(m.layers) && __ldg(m.srcBeta + size_t(min(l, int(m.layers) - 1)) * m.T + t) > 0.0f;
-        J[g] = 0.0f;
-        lnR[g] = 0.0f;
-        kf[g] = kImg > l ? float(l + 1 - kImg) : float(kImg - l);
-        lrow[g] = l * int(m.T);
-        rstep[g] = kImg > l ? int(m.T) : -int(m.T);
-        left[g] = expectedReflections(j);
-        const float ic = D2 / (float(l - kImg) + 0.5f);
-        invc[g] = kImg > l ? ic : -ic;
+// The lines' table: per triangle the gain along z in the unfolded direction a
+// line moves in.  Entry i of triangle t belongs to the i-th layer of the
+// sequence down, up, down (phases x layers entries, i falling along a line's
+// way: phase 0 is a line moving down in layer i, phase 1 one moving up in
+// layer 2 layers - 1 - i, phase 2 down again) and holds (F, g): g of the layer's
+// prism (beta A - B, -claddingAbsorption in cladding) and F = the integral of g
+// over the sequence up to the middle of the entry, in level units, summed in
+// FP64 and centred so that its FP32 rounding is small.  A line's integral over
+// any stretch of a triangle is then a difference of two F + g (position -
+// middle), whatever the number of levels and reflections in between.
+// Without reflections a line stays in phase 0 or 1 (phases = 2).
+__global__ void lineTableKernel(const float* gainBeta, float A, float B, float cladAbs, uint32_t T, uint32_t layers,
+                                uint32_t phases, float2* line) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    double total = 0.0;
+    for (uint32_t l = 0; l < layers; ++l) {
+        const float b = gainBeta[size_t(l) * T + t];
+        total += double((b == b) ? fmaf(b, A, -B) : -fminf(cladAbs, 1e30f));  // finite: F is a difference
     }
-    GlobalLoader load{m.walk};
-    uint32_t tk = t;
-    float sc = D2;
-    bool done = false;
-    for (int step = 0; step < kMaxSteps && !done; ++step) {
-        float4 a, b, cc;
-        load(tk, a, b, cc);
-        float bn = -1.0f, bd = 0.0f;
-        int bw = -1;
-        const auto edge = [&](float nx, float ny, float ce, int nbw) {
-            const float dd = -fmaf(nx, ux, ny * uy);
-            const float nm = fmaf(nx, S.x, fmaf(ny, S.y, -ce));
-            const bool okE = dd > 0.0f;  // the entry edge has dd < 0, a boundary edge NaN (see stepRay)
-            if (okE && nm * bd > bn * dd) {
-                bn = nm;
-                bd = dd;
-                bw = nbw;
-            }
-        };
-        edge(a.x, a.y, a.z, __float_as_int(cc.y));
-        edge(a.w, b.x, b.y, __float_as_int(cc.z));
-        edge(b.z, b.w, cc.x, __float_as_int(cc.w));
-        float sOut = fmaxf(fminf(__fdividef(bn, bd), sc), 0.0f);
-        if (sOut <= m.tolEnd) {
-            sOut = 0.0f;
-            done = true;
-        }
-        // beta of every line's current prism in this triangle, issued together
-        float gbv[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) gbv[g] = ok[g] ? __ldg(gcol + uint32_t(lrow[g]) + tk) : 0.0f;
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            if (!ok[g]) continue;
-            float s = sc;
-            float gb = gbv[g];
-            while (true) {
-                const float sb = kf[g] * invc[g];
-                if (!(sb > sOut)) break;
-                J[g] = fmaf(TAB ? gb : ((gb == gb) ? fmaf(gb, L.A, -L.B) : -m.cladAbs), s - sb, J[g]);
-                s = sb;
-                const int cand = lrow[g] + rstep[g];
-                if (uint32_t(cand) >= m.P) {  // a physical bottom/top surface: reflect
-                    if (left[g] <= 0) {
-                        ok[g] = false;
-                        break;
-                    }
-                    const float dz = (float(l0 + g - kImg) + 0.5f) * m.h;
-                    const float uz = dz * rsqrtf(fmaf(D2, D2, dz * dz));
-                    lnR[g] += __logf(reflectFactor(m, tk, cand < 0 ? 0 : 1, uz));
-                    --left[g];
-                    rstep[g] = -rstep[g];
-                } else {
-                    lrow[g] = cand;
-                    gb = __ldg(gcol + uint32_t(cand) + tk);
-                }
-                kf[g] += 1.0f;
-            }
-            if (!ok[g]) continue;
-            J[g] = fmaf(TAB ? gb : ((gb == gb) ? fmaf(gb, L.A, -L.B) : -m.cladAbs), s - sOut, J[g]);
-        }
-        if (!done) {
-            tk = uint32_t(bw) >> 2;
-            sc = sOut;
-        }
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const int l = l0 + g;
-        if (l >= int(m.layers)) continue;
-        float v = -INFINITY;
-        if (ok[g] && done) {
-            const float dz = (float(l - kImg) + 0.5f) * m.h;
-            const float D3sq = fmaf(D2, D2, dz * dz);
-            if (left[g] > 0) {  // the bounce happens at the target itself, in the final triangle
-                lnR[g] += __logf(reflectFactor(m, tk, lrow[g] + rstep[g] < 0 ? 0 : 1, dz * rsqrtf(D3sq)));
-            }
-            const float beta = __ldg(m.srcBeta + size_t(l) * m.T + t);
-            v = __logf(beta * area * m.h / D3sq) + J[g] * (sqrtf(D3sq) * inv2) + lnR[g];
-        }
-        out[size_t(l) * m.T] = v;
+    float2* out = line + size_t(t) * phases * layers;
+    double F = -0.5 * double(phases) * total;
+    for (uint32_t i = 0; i < phases * layers; ++i) {
+        const uint32_t r = i % layers, l = (i / layers) & 1u ? layers - 1u - r : r;
+        const float b = gainBeta[size_t(l) * T + t];
+        const float g = (b == b) ? fmaf(b, A, -B) : -fminf(cladAbs, 1e30f);
+        out[i] = make_float2(float(F + 0.5 * double(g)), g);
+        F += double(g);
     }
 }
 
-// Line-team importance kernel: a team of TL lanes per (sample row,
-// triangle t).  Every line from the centre of a prism (t, l) to an image
-// s_j of the sample point projects onto the same 2-D segment, centroid ->
-// sample point, so the team walks that segment in lock step (no divergence
-// in the number of triangles crossed) and each lane carries LPL of the
-// triangle's slices x layers lines through the level planes and
-// reflections of every triangle on it (teams of TL lanes, lines in chunks
-// of TL x LPL).  The 2-D edge tests are thus shared by up to TL x LPL lines
-// instead of the G of importanceKernel; the per-line arithmetic is
-// importanceKernel's, operation for operation, so the weights are the same
-// bits.  COUNT: also add the walk's crossings (triangle segments plus level
-// planes and reflections, per line) to *L.crossings.
-template <int TL, int LPL, bool TAB = false, bool COUNT = false>
+__host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slices == 1 ? 2u : 3u; }
+
+// Line-team importance kernel: a team of TL lanes per (sample point,
+// triangle t).  Every line from the centre of a prism (t, l) to an image of a
+// sample point projects onto the same 2-D segment, centroid -> sample point,
+// whatever its layer, its reflection slice and the sample's level, so the
+// team walks that segment once for all of them -- the slices x layers lines of
+// every requested level of the point -- in lock step, LPL lines per lane
+// (chunks of TL x LPL lines), sharing the 2-D edge tests (stepRay's windows).
+// ln w = ln(beta V / d^2) + Int g dl.
+// A line crosses a level every D2 / |l + 1/2 - kImg| along the segment; at
+// distance s, n = floor of the levels left to its image level, so its
+// table entry is n + base.  Per triangle and line: the entry and the position
+// in it at the exit (one FFMA, one rounding by 1.5 2^23, two adds), one table
+// load at the entry and one at the exit, and five operations for the
+// integral.  Stepping through the levels one by one cost a loop per line that
+// the warp ran as often as its steepest line needed (216 warp instructions per
+// triangle for 96 lines).
+// A bounce is only an event (the branch) for its factor, which a line beyond
+// the critical angle does not have, and for the second bounce of slice 4, which
+// leaves the table's sequence at phase 0 for phase 1.
+// Precision: F's rounding enters only where the entry changes, so a nearly
+// level line stays as exact as the sum of its segments.
+// COUNT: also add the walk's crossings (triangle segments plus level planes
+// and reflections, per line) to *L.crossings.
+template <int TL, int LPL, bool COUNT = false>
 __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) {
     static_assert(TL >= 1 && TL <= 32 && (32 % TL) == 0, "a team is a power-of-two part of a warp");
     const MeshView& m = L.m;
-    const float* gcol = TAB ? m.gTab : m.gainBeta;
     constexpr uint32_t kTeams = 256 / TL;
+    constexpr float kRound = 12582912.0f;   // 1.5 2^23: adding it rounds to an integer
+    constexpr int kRoundBits = 0x4B400000;
     const uint32_t tIdx = blockIdx.x * kTeams + threadIdx.x / TL;  // triangle (or candidate) of the team
     const uint32_t li = threadIdx.x % TL;
-    const uint32_t row = L.rowList ? L.rowList[blockIdx.y] : blockIdx.y;
+    const uint32_t row0 = L.rowList ? L.rowList[blockIdx.y] : blockIdx.y;
     const uint32_t strideL = L.cand ? L.K : m.T;            // entries per layer of a slice
     unsigned long long counted = 0;
-    if (tIdx < strideL && !(L.rowFlag && !L.rowFlag[L.flagBase + row])) {
-        const uint32_t sample = L.firstSample + row;
-        const uint32_t pt = sample % m.Np;
+    if (tIdx < strideL && !(L.rowFlag && !L.rowFlag[L.flagBase + row0])) {
+        const int layers = int(m.layers);
+        const uint32_t sample0 = L.firstSample + row0;
+        const int ls0 = int(sampleLevel(m, sample0));
+        const uint32_t pt = sample0 - uint32_t(ls0) * m.Np;
         const uint32_t t = L.cand ? __ldg(L.cand + size_t(pt) * L.K + tIdx) : tIdx;
         const float2 S = __ldg(m.points + pt);
-        const int ls = int(sample / m.Np);
         const float2 c = __ldg(m.centroid + t);
         const float area = __ldg(&m.geo[2 * t + 1].z);
         const float dx = c.x - S.x, dy = c.y - S.y;
         const float D2 = sqrtf(fmaf(dx, dx, dy * dy));
         const float inv2 = 1.0f / D2;
         const float ux = dx * inv2, uy = dy * inv2;
-        float* outRow = L.lnw + size_t(row) * L.nW + tIdx;
         const size_t strideJ = size_t(strideL) * m.layers;
-        const uint32_t nLines = L.slices * m.layers;
+        const uint32_t stride = linePhases(L.slices) * m.layers;
+        // rows of the point: row0, row0 + Np, ... (listed and flagged rows one by one)
+        const uint32_t levels = L.rowList || L.rowFlag ? 1u : 1u + (L.rows - 1u - row0) / m.Np;
+        const uint32_t nLines = levels * L.slices * m.layers;
+        const float2* edge = reinterpret_cast<const float2*>(m.win + 4 * size_t(t));
+        const float2 n0e = __ldg(edge), n1e = __ldg(edge + 2);
+        const uint32_t firstWindow =
+            4 * t + (!(-fmaf(n0e.x, ux, n0e.y * uy) > 0.0f) ? 1u : (!(-fmaf(n1e.x, ux, n1e.y * uy) > 0.0f) ? 2u : 0u));
         for (uint32_t c0 = 0; c0 < nLines; c0 += TL * LPL) {
-            float J[LPL], lnR[LPL], invc[LPL], nextPlane[LPL];
-            float kf[LPL];  // as in importanceKernel
-            int lrow[LPL], rstep[LPL], left[LPL], kImg[LPL], lay[LPL];  // lrow, rstep: as in importanceKernel
-            uint32_t sl[LPL];
-            bool ok[LPL];
-            const uint16_t* order = m.lineOrder[L.slices == 5 ? 1 : 0];
-#pragma unroll
-            for (int g = 0; g < LPL; ++g) {
+            // per line: levels per unit of s, the integral in level units, the
+            // bounces' ln factor, the position in the current entry relative to
+            // its middle, the current entry and its offset from n, n at the next
+            // event (-1: none), and the bounces (low bits: surface, more, slice 4)
+            float inv[LPL], acc[LPL], lnR[LPL], f[LPL], nEvent[LPL];
+            int entry[LPL], base[LPL], bounce[LPL];
+            const auto lineOf = [&](int g, int& l, uint32_t& j, int& ls) {
                 const uint32_t qq = c0 + li + uint32_t(TL * g);
                 const bool valid = qq < nLines;
-                const uint32_t q = valid && order ? uint32_t(__ldg(order + size_t(ls) * nLines + qq)) : qq;
-                const uint32_t l = valid ? q / L.slices : 0u;
-                const uint32_t j = valid ? q - l * L.slices : 0u;
-                sl[g] = valid ? j : 0xffffffffu;
-                lay[g] = int(l);
-                kImg[g] = imageLevel(ls, int(m.layers), j);
-                ok[g] = valid && __ldg(m.srcBeta + size_t(l) * m.T + t) > 0.0f;
-                J[g] = 0.0f;
+                const uint32_t q = valid ? qq : 0u;
+                const uint32_t x = uint32_t((uint64_t(q) * L.divLm) >> L.divLs);
+                const uint32_t lev = L.slices == 1 ? x : x / 5u;
+                l = int(q - x * m.layers);
+                j = L.slices == 1 ? 0u : x - 5u * lev;
+                ls = ls0 + int(lev);
+                return valid;
+            };
+#pragma unroll
+            for (int g = 0; g < LPL; ++g) {
+                int l, ls;
+                uint32_t j;
+                lineOf(g, l, j, ls);
+                const int kImg = imageLevel(ls, layers, j);
+                const float a = fabsf(float(l - kImg) + 0.5f);
+                inv[g] = a * inv2;
+                acc[g] = 0.0f;
                 lnR[g] = 0.0f;
-                kf[g] = kImg[g] > int(l) ? float(int(l) + 1 - kImg[g]) : float(kImg[g] - int(l));
-                lrow[g] = int(l * m.T);
-                rstep[g] = kImg[g] > int(l) ? int(m.T) : -int(m.T);
-                left[g] = expectedReflections(j);
-                const float ic = D2 / (float(int(l) - kImg[g]) + 0.5f);
-                invc[g] = kImg[g] > int(l) ? ic : -ic;
-                // sigma of the next level plane toward the image level (carried,
-                // recomputed only when the line crosses it)
-                nextPlane[g] = kf[g] * invc[g];
+                f[g] = 0.0f;
+                const bool up = j == 0 ? kImg > l : (j == 1 || j == 4);  // the line's last direction
+                const int b = j == 4 ? -ls : (up ? 2 * layers - ls : ls);
+                entry[g] = (kImg > l ? kImg - l - 1 : l - kImg) + b;
+                base[g] = b - kRoundBits;
+                nEvent[g] = -1.0f;
+                bounce[g] = 0;
+                if (j > 0) {
+                    const float dz = (float(l - kImg) + 0.5f) * m.h;
+                    const float uz = dz * rsqrtf(fmaf(D2, D2, dz * dz));
+                    const bool needB = !(uz * uz <= m.tirCos2[0]), needT = !(uz * uz <= m.tirCos2[1]);
+                    const bool bottomFirst = j == 1 || j == 3;
+                    bounce[g] = (bottomFirst ? 0 : 1) | (j >= 3 ? 2 : 0) | (needB ? 4 : 0) | (needT ? 8 : 0) |
+                                (j == 4 ? 16 : 0);
+                    if (j == 4 || (bottomFirst ? needB : needT) || (j == 3 && needT))
+                        nEvent[g] = float(j == 1 ? ls : (j == 2 ? layers - ls : (j == 3 ? 2 * layers - ls : layers + ls)));
+                }
             }
-            GlobalLoader load{m.walk};
-            uint32_t tk = t;
+            uint32_t w = firstWindow;
+            float4 wa = __ldg(m.win + w), wb = __ldg(m.win + w + 1);
+            uint32_t columns = 0;
             float sc = D2;
             bool done = false;
             for (int step = 0; step < kMaxSteps && !done; ++step) {
-                float4 a, b, cc;
-                load(tk, a, b, cc);
-                float bn = -1.0f, bd = 0.0f;
-                int bw = -1;
-                const auto edge = [&](float nx, float ny, float ce, int nbw) {
-                    const float dd = -fmaf(nx, ux, ny * uy);
-                    const float nm = fmaf(nx, S.x, fmaf(ny, S.y, -ce));
-                    const bool okE = dd > 0.0f;  // the entry edge has dd < 0, a boundary edge NaN (see stepRay)
-                    if (okE && nm * bd > bn * dd) {
-                        bn = nm;
-                        bd = dd;
-                        bw = nbw;
-                    }
-                };
-                edge(a.x, a.y, a.z, __float_as_int(cc.y));
-                edge(a.w, b.x, b.y, __float_as_int(cc.z));
-                edge(b.z, b.w, cc.x, __float_as_int(cc.w));
-                float sOut = fmaxf(fminf(__fdividef(bn, bd), sc), 0.0f);
-                if (sOut <= m.tolEnd) {
-                    sOut = 0.0f;
-                    done = true;
-                }
-                float gbv[LPL];
+                const uint32_t tk = w >> 2;
+                const float2* col = L.line + size_t(tk) * stride;
+                float2 in[LPL];
 #pragma unroll
-                for (int g = 0; g < LPL; ++g) gbv[g] = ok[g] ? __ldg(gcol + uint32_t(lrow[g]) + tk) : 0.0f;
+                for (int g = 0; g < LPL; ++g) in[g] = __ldg(col + entry[g]);
+                const float q1 = edgeExit(wa, ux, uy, S.x, S.y), q2 = edgeExit(wb, ux, uy, S.x, S.y);
+                const float qm = fmaxf(q1, q2);
+                const uint32_t code = __float_as_uint(q2 == qm ? wb.w : wa.w);
+                wa = __ldg(m.win + code);
+                wb = __ldg(m.win + code + 1);
+                float sOut = fminf(qm, sc);
+                done = !(sOut > m.tolEnd);
+                sOut = done ? 0.0f : sOut;
+                if (COUNT) ++columns;
 #pragma unroll
                 for (int g = 0; g < LPL; ++g) {
-                    if (!ok[g]) continue;
-                    if (COUNT) ++counted;
-                    float s = sc;
-                    float gb = gbv[g];
-                    while (true) {
-                        const float sb = nextPlane[g];
-                        if (!(sb > sOut)) break;
-                        if (COUNT) ++counted;
-                        J[g] = fmaf(TAB ? gb : ((gb == gb) ? fmaf(gb, L.A, -L.B) : -m.cladAbs), s - sb, J[g]);
-                        s = sb;
-                        const int cand = lrow[g] + rstep[g];
-                        if (uint32_t(cand) >= m.P) {  // a physical bottom/top surface: reflect
-                            if (left[g] <= 0) {
-                                ok[g] = false;
-                                break;
-                            }
-                            const float dz = (float(lay[g] - kImg[g]) + 0.5f) * m.h;
-                            const float uz = dz * rsqrtf(fmaf(D2, D2, dz * dz));
-                            lnR[g] += __logf(reflectFactor(m, tk, cand < 0 ? 0 : 1, uz));
-                            --left[g];
-                            rstep[g] = -rstep[g];
+                    const float p = fmaf(sOut, inv[g], -0.5f);
+                    const float r = p + kRound;
+                    const float n = r - kRound;  // levels left at the exit
+                    const float fo = p - n;
+                    while (n < nEvent[g]) {  // a bounce on the way
+                        const int s = bounce[g] & 1;
+                        if (bounce[g] & (4 << s)) lnR[g] += __logf(m.reflect ? __ldg(m.reflect + 2 * tk + s) : 0.0f);
+                        if (bounce[g] & 2) {
+                            bounce[g] = (bounce[g] & ~2) ^ 1;
+                            nEvent[g] -= float(layers);
                         } else {
-                            lrow[g] = cand;
-                            gb = __ldg(gcol + uint32_t(cand) + tk);
+                            if (bounce[g] & 16) {  // the second bounce of slice 4: from entry 0 to 2 layers - 1
+                                base[g] += 2 * layers;
+                                acc[g] += __ldg(&col[2 * layers].x) - __ldg(&col[0].x);
+                            }
+                            nEvent[g] = -1.0f;
                         }
-                        kf[g] += 1.0f;
-                        nextPlane[g] = kf[g] * invc[g];
                     }
-                    if (!ok[g]) continue;
-                    J[g] = fmaf(TAB ? gb : ((gb == gb) ? fmaf(gb, L.A, -L.B) : -m.cladAbs), s - sOut, J[g]);
+                    entry[g] = __float_as_int(r) + base[g];
+                    const float2 out = __ldg(col + entry[g]);
+                    acc[g] += fmaf(in[g].y, f[g], fmaf(-out.y, fo, in[g].x - out.x));
+                    f[g] = fo;
                 }
                 if (!done) {
-                    tk = uint32_t(bw) >> 2;
+                    w = code;
                     sc = sOut;
                 }
             }
+            const uint32_t tk = w >> 2;  // the target's triangle
 #pragma unroll
             for (int g = 0; g < LPL; ++g) {
-                if (sl[g] == 0xffffffffu) continue;
-                const int l = lay[g];
+                int l, ls;
+                uint32_t j;
+                if (!lineOf(g, l, j, ls)) continue;
+                const int kImg = imageLevel(ls, layers, j);
+                const float beta = __ldg(m.srcBeta + size_t(l) * m.T + t);
                 float v = -INFINITY;
-                if (ok[g] && done) {
-                    const float dz = (float(l - kImg[g]) + 0.5f) * m.h;
-                    const float D3sq = fmaf(D2, D2, dz * dz);
-                    if (left[g] > 0) {  // the bounce happens at the target itself, in the final triangle
-                        lnR[g] += __logf(reflectFactor(m, tk, lrow[g] + rstep[g] < 0 ? 0 : 1, dz * rsqrtf(D3sq)));
+                if (beta > 0.0f) {
+                    const float a = fabsf(float(l - kImg) + 0.5f);
+                    if (COUNT) counted += columns + uint32_t(a - 0.5f);
+                    if (done) {
+                        const float dz = (float(l - kImg) + 0.5f) * m.h;
+                        const float D3sq = fmaf(D2, D2, dz * dz);
+                        float ln = lnR[g];
+                        // the bounce happens at the target itself, in the final triangle
+                        if (j > 0 && ls == (j == 1 || j == 4 ? 0 : layers))
+                            ln += __logf(reflectFactor(m, tk, j == 1 || j == 4 ? 0 : 1, dz * rsqrtf(D3sq)));
+                        v = __logf(beta * area * m.h / D3sq) + acc[g] * (sqrtf(D3sq) / a) + ln;
                     }
-                    const float beta = __ldg(m.srcBeta + size_t(l) * m.T + t);
-                    v = __logf(beta * area * m.h / D3sq) + J[g] * (sqrtf(D3sq) * inv2) + lnR[g];
                 }
-                outRow[size_t(sl[g]) * strideJ + size_t(l) * strideL] = v;
+                L.lnw[size_t(row0 + uint32_t(ls - ls0) * m.Np) * L.nW + size_t(j) * strideJ + size_t(l) * strideL + tIdx] = v;
             }
         }
     }
@@ -419,51 +346,45 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
     }
 }
 
-// Team width of the line-team kernel: the narrowest team whose lanes hold a
-// sample's slices x layers lines of one triangle in one chunk of 3 per lane
-// (32 lanes: chunks of 96 lines).
-uint32_t importanceTeamWidth(uint32_t lines) {
-    return lines <= 12 ? 4u : lines <= 24 ? 8u : lines <= 48 ? 16u : 32u;
-}
-
-// The importance walks of `rows` sample rows: layers = 0 (the library's
-// choice): importanceTeamKernel; 2, 4 or 8: importanceKernel with that many
-// prism layers per thread.  tab: il.m.gTab holds g for il.A, il.B.  count:
-// the counting team kernel (il.crossings accumulates the walk's crossings).
-cudaError_t launchImportance(uint32_t layers, const ImportanceLaunch& il, uint32_t meshLayers, uint32_t T,
-                             uint32_t rows, cudaStream_t stream, bool tab = false, bool count = false) {
-    if (layers == 0 || count || il.cand) {
-        const uint32_t tl = importanceTeamWidth(il.slices * meshLayers);
-        const uint32_t nTri = il.cand ? il.K : T;
-#define HASE_TEAM(TL)                                                                         \
-    {                                                                                         \
-        const dim3 grid((nTri + 256 / TL - 1) / (256 / TL), rows);                            \
-        if (count) importanceTeamKernel<TL, 3, false, true><<<grid, 256, 0, stream>>>(il);   \
-        else if (tab) importanceTeamKernel<TL, 3, true><<<grid, 256, 0, stream>>>(il);       \
-        else importanceTeamKernel<TL, 3><<<grid, 256, 0, stream>>>(il);                      \
+// The importance walks of `rows` sample rows (il.rowList: that many listed
+// rows).  A point's lines -- its requested levels x slices x layers -- fill the
+// narrowest team that holds them with at most 4 per lane, in as few chunks of
+// a full warp as there must be; the lines per lane then as even as they go.
+// count: the counting kernel (il.crossings accumulates the walk's crossings).
+cudaError_t launchImportance(ImportanceLaunch il, uint32_t meshLayers, uint32_t T, uint32_t Np, uint32_t rows,
+                             cudaStream_t stream, bool count = false) {
+    il.rows = rows;
+    invariantDivisor(meshLayers, il.divLm, il.divLs);
+    const bool single = il.rowList || il.rowFlag;
+    const uint32_t gridRows = single ? rows : std::min(rows, Np);
+    const uint64_t lines = uint64_t(il.slices) * meshLayers * (single ? 1u : (rows + Np - 1) / Np);
+    const uint32_t nTri = il.cand ? il.K : T;
+    const uint32_t tl = lines <= 16 ? 4u : lines <= 32 ? 8u : lines <= 64 ? 16u : 32u;
+    const uint64_t chunks = (lines + 4 * tl - 1) / (4 * tl);
+    const uint32_t lpl = uint32_t((lines + tl * chunks - 1) / (tl * chunks));
+#define HASE_TEAM(TL, LPL)                                                            \
+    {                                                                                 \
+        const dim3 grid((nTri + 256 / TL - 1) / (256 / TL), gridRows);                \
+        importanceTeamKernel<TL, LPL><<<grid, 256, 0, stream>>>(il);                  \
     }
-        switch (tl) {
-            case 4: HASE_TEAM(4) break;
-            case 8: HASE_TEAM(8) break;
-            case 16: HASE_TEAM(16) break;
-            default: HASE_TEAM(32) break;
+    if (count) {
+        const dim3 grid((nTri + 7) / 8, gridRows);
+        importanceTeamKernel<32, 3, true><<<grid, 256, 0, stream>>>(il);
+    } else if (tl == 4) {
+        switch (lpl) {
+            case 1: HASE_TEAM(4, 1) break;
+            case 2: HASE_TEAM(4, 2) break;
+            case 3: HASE_TEAM(4, 3) break;
+            default: HASE_TEAM(4, 4) break;
         }
-#undef HASE_TEAM
-        return cudaGetLastError();
-    }
-    const uint32_t G = layers;
-    const uint32_t threads = il.slices * ((meshLayers + G - 1) / G) * T;
-    const dim3 grid((threads + 255) / 256, rows);
-    if (G == 2) {
-        if (tab) importanceKernel<2, true><<<grid, 256, 0, stream>>>(il);
-        else importanceKernel<2><<<grid, 256, 0, stream>>>(il);
-    } else if (G == 8) {
-        if (tab) importanceKernel<8, true><<<grid, 256, 0, stream>>>(il);
-        else importanceKernel<8><<<grid, 256, 0, stream>>>(il);
+    } else if (tl == 8) {
+        if (lpl <= 3) HASE_TEAM(8, 3) else HASE_TEAM(8, 4)
+    } else if (tl == 16) {
+        if (lpl <= 3) HASE_TEAM(16, 3) else HASE_TEAM(16, 4)
     } else {
-        if (tab) importanceKernel<4, true><<<grid, 256, 0, stream>>>(il);
-        else importanceKernel<4><<<grid, 256, 0, stream>>>(il);
+        if (lpl <= 3) HASE_TEAM(32, 3) else HASE_TEAM(32, 4)
     }
+#undef HASE_TEAM
     return cudaGetLastError();
 }
 
@@ -1881,20 +1802,9 @@ __global__ void gainTableKernel(const float* gainBeta, float A, float B, float c
 }
 
 // -------------------------------------------------------- host side ----
-// Multiplier and shift with floor(n / d) = (n * mul) >> shift for every
-// n < 2^31 and 1 <= d < 2^32 (Granlund and Montgomery, "Division by invariant
-// integers using multiplication", PLDI 1994, theorem 4.2 with N = 31):
-// l = ceil(log2 d), mul = ceil(2^(31 + l) / d) (< 2^32), shift = 31 + l.
-void invariantDivisor(uint32_t d, uint32_t& mul, uint32_t& shift) {
-    uint32_t l = 0;
-    while ((uint64_t(1) << l) < d) ++l;
-    shift = 31 + l;
-    mul = uint32_t(((uint64_t(1) << shift) + d - 1) / d);
-}
-
 struct HostTables {
     std::vector<int4> verts;
-    std::vector<float4> tri, walk, win, geo;
+    std::vector<float4> tri, win, geo;
     std::vector<float2> centroid, points;
 };
 
@@ -1960,35 +1870,22 @@ hase_status buildHostTables(const hase_mesh_desc* d, HostTables& h, double& exte
         float* rec = &h.tri[3 * t + 2].y;
         std::memcpy(rec, w, sizeof(w));
     }
-    // the walks' copy: a boundary edge's normal is NaN, so its dd > 0 test fails
-    // and the walks need no separate boundary test
-    h.walk = h.tri;
-    const float nan = std::numeric_limits<float>::quiet_NaN();
-    for (uint32_t t = 0; t < T; ++t) {
-        float* r = &h.walk[3 * size_t(t)].x;  // nx0 ny0 c0 nx1 | ny1 c1 nx2 ny2 | c2 nb0 nb1 nb2
-        static const int kNx[3] = {0, 3, 6}, kNy[3] = {1, 4, 7};
-        for (int e = 0; e < 3; ++e) {
-            int32_t nb;
-            std::memcpy(&nb, r + 9 + e, sizeof(nb));
-            if (nb < 0) r[kNx[e]] = r[kNy[e]] = nan;
-        }
-    }
-    // the ray walk's windows: the same edges in the slots e0 e1 e2 e0
+    // the walks' windows: the same edges in the slots e0 e1 e2 e0
     h.win.resize(4 * size_t(T));
     for (uint32_t t = 0; t < T; ++t) {
-        const float* r = &h.walk[3 * size_t(t)].x;
+        const float* r = &h.tri[3 * size_t(t)].x;  // nx0 ny0 c0 nx1 | ny1 c1 nx2 ny2 | c2 nb0 nb1 nb2
+        float4* w = &h.win[4 * size_t(t)];
         for (int e = 0; e < 3; ++e) {
-            int32_t nb;
-            std::memcpy(&nb, r + 9 + e, sizeof(nb));
-            float4& w = h.win[4 * size_t(t) + e];
-            w = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
-            if (nb < 0) continue;
-            static const int kAt[3] = {0, 3, 6};
-            const uint32_t code = (uint32_t(nb) & ~3u) | windowSlot(uint32_t(nb) & 3u);
-            w = make_float4(r[kAt[e]], r[kAt[e] + 1], r[kAt[e] + 2], 0.0f);
-            std::memcpy(&w.w, &code, sizeof(code));
+            const int32_t o = nbr[3 * t + e];
+            if (o < 0) {
+                w[e] = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+                continue;
+            }
+            const uint32_t code = (uint32_t(o / 3) << 2) | windowSlot(uint32_t(o % 3));
+            w[e] = make_float4(r[3 * e], r[3 * e + 1], r[3 * e + 2], 0.0f);
+            std::memcpy(&w[e].w, &code, sizeof(code));
         }
-        h.win[4 * size_t(t) + 3] = h.win[4 * size_t(t)];
+        w[3] = w[0];
     }
     return HASE_OK;
 }
@@ -2198,27 +2095,6 @@ void buildFarCells(const std::vector<float2>& centroid, std::vector<uint32_t>& c
     }
 }
 
-// The importance kernel's line order: for every sample level ls, the lines
-// q = l * slices + j (layer l, reflection slice j) by increasing distance
-// |l + 1/2 - kImg| to the image level (ties by q).  A line crosses about that
-// many level planes along its 2-D path, so the lines of one lane slot of a
-// team cross similar numbers of planes per triangle.
-void buildLineOrder(uint32_t layers, uint32_t slices, std::vector<uint16_t>& ord) {
-    const uint32_t n = slices * layers;
-    ord.resize(size_t(layers + 1) * n);
-    std::vector<std::pair<double, uint32_t>> key(n);
-    for (uint32_t ls = 0; ls <= layers; ++ls) {
-        for (uint32_t q = 0; q < n; ++q) {
-            const uint32_t l = q / slices, j = q % slices;
-            const int L = int(layers), s = int(ls);
-            const int kImg = j == 1 ? -s : j == 2 ? 2 * L - s : j == 3 ? s - 2 * L : j == 4 ? s + 2 * L : s;
-            key[q] = {std::fabs(double(l) + 0.5 - double(kImg)), q};
-        }
-        std::sort(key.begin(), key.end());
-        for (uint32_t i = 0; i < n; ++i) ord[size_t(ls) * n + i] = uint16_t(key[i].second);
-    }
-}
-
 }  // namespace
 
 struct hase_context {
@@ -2233,9 +2109,9 @@ struct hase_context {
     std::vector<double> betaCells, sigmaA, sigmaE;
     bool hasReflect = false;
     float tirCos2[2] = {-1.0f, -1.0f};
-    DevBuf<float4> tri, walk, win, geo;
+    DevBuf<float4> tri, win, geo;
     DevBuf<int4> verts;
-    DevBuf<uint16_t> lineOrder[2];  // importance line order per sample level: 1 and 5 reflection slices
+    DevBuf<float2> line;  // the importance lines' table of the last solve (lineTableKernel)
     // local proposal (hase_context_set_local_proposal): per point the K
     // triangles nearest to it (by centroid distance, nearest first) and the
     // same set by ascending index; the far proposal's prefix of beta V over
@@ -2289,7 +2165,6 @@ struct hase_context {
         invariantDivisor(T, v.divTm, v.divTs);
         invariantDivisor(Np, v.divNpm, v.divNps);
         v.tri = tri.p;
-        v.walk = walk.p;
         v.win = win.p;
         v.geo = geo.p;
         v.verts = verts.p;
@@ -2299,8 +2174,6 @@ struct hase_context {
         v.srcBeta = srcBeta.p;
         v.points = points.p;
         v.reflect = hasReflect ? reflect.p : nullptr;
-        v.lineOrder[0] = lineOrder[0].p;
-        v.lineOrder[1] = lineOrder[1].p;
         v.T = T;
         v.layers = layers;
         v.P = P;
@@ -2447,6 +2320,17 @@ void localFields(hase_context* c, ImportanceLaunch& il) {
     if (!c->localK) return;
     il.cand = c->candTri.p;
     il.K = c->localK;
+}
+
+// The importance lines' table of the context's beta for the averaged (A, B),
+// built on stream s.
+hase_status buildLineTable(hase_context* c, double A, double B, uint32_t slices, cudaStream_t s) {
+    const uint32_t phases = linePhases(slices);
+    HASE_CUDA(c->line.ensure(size_t(c->P) * phases));
+    lineTableKernel<<<(c->T + 127) / 128, 128, 0, s>>>(c->gainBeta.p, float(A), float(B), float(c->cladAbs), c->T,
+                                                       c->layers, phases, c->line.p);
+    HASE_CUDA(cudaGetLastError());
+    return HASE_OK;
 }
 
 struct LearnedArgs {
@@ -2724,17 +2608,9 @@ hase_status hase_context_create(const hase_mesh_desc* d, const hase_spectrum_des
         return HASE_OK;
     };
     if ((st = up(c->tri, ht.tri)) != HASE_OK) return cleanup(st);
-    if ((st = up(c->walk, ht.walk)) != HASE_OK) return cleanup(st);
     if ((st = up(c->win, ht.win)) != HASE_OK) return cleanup(st);
     if ((st = up(c->geo, ht.geo)) != HASE_OK) return cleanup(st);
     if ((st = up(c->verts, ht.verts)) != HASE_OK) return cleanup(st);
-    if (uint64_t(5) * c->layers < 65536) {  // importance line order (16-bit line indices)
-        for (int r = 0; r < 2; ++r) {
-            std::vector<uint16_t> ord;
-            buildLineOrder(c->layers, r ? 5u : 1u, ord);
-            if ((st = up(c->lineOrder[r], ord)) != HASE_OK) return cleanup(st);
-        }
-    }
     if ((st = up(c->centroid, ht.centroid)) != HASE_OK) return cleanup(st);
     if ((st = up(c->points, ht.points)) != HASE_OK) return cleanup(st);
     if (c->gainBeta.ensure(c->P) != cudaSuccess || c->srcBeta.ensure(c->P) != cudaSuccess)
@@ -2923,15 +2799,17 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     std::vector<double> hRse;
     std::vector<uint32_t> hTot;
 
-    // the importance walks, and the ray walk of a monochromatic solve, read
-    // each prism's g from a table (rebuilt here: beta may have changed since
-    // the last solve)
+    // the ray walk of a monochromatic solve and the far prior read each
+    // prism's g from a table, the importance walks their lines' integrals
+    // (rebuilt here: beta may have changed since the last solve)
     // walk mode of the ray launches (the logging launches keep the general walk)
     const int walk = logOut ? kWalkBeta : (nLambda == 1 ? kWalkTable : (c->hasClad ? kWalkBeta : kWalkBetaNoClad));
     HASE_CUDA(c->gTab.ensure(c->P));
     gainTableKernel<<<(c->P + 255) / 256, 256, 0, c->stream>>>(c->gainBeta.p, float(meanA), float(meanB),
                                                                float(c->cladAbs), c->P, c->gTab.p);
     HASE_CUDA(cudaGetLastError());
+    const bool walks = la ? la->fallbackVariance > 0.0f : !gridWeights;
+    if (walks) HASE_TRY(buildLineTable(c, meanA, meanB, slices, c->stream));
     ProposalView fpv{};
     if (farPrior) {  // the far prior's cell gains for this solve's g, and the layer-averaged coarse gain grid
         const uint32_t n = c->farCells * c->layers;
@@ -2957,18 +2835,18 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     res->totalMilliseconds = 0;
     res->passes = 0;
     res->unconvergedSamples = 0;
-    res->kernelLaunches = farPrior ? 3 : 1;  // the gain table (and the far prior's cell gains and gain grid)
+    res->kernelLaunches = (farPrior ? 3 : 1) + (walks ? 1 : 0);  // the tables (and the far prior's cell gains and gain grid)
     uint64_t droppedTotal = 0;
 
     for (uint32_t b0 = 0; b0 < nS; b0 += rows) {
         const uint32_t nRows = std::min(rows, nS - b0);
         const uint32_t firstSample = first + b0;
         HASE_CUDA(cudaEventRecord(c->ev[0], c->stream));
-        ImportanceLaunch il{mv, firstSample, slices, nW, float(meanA), float(meanB), c->lnw.p, nullptr};
+        ImportanceLaunch il{mv, firstSample, nRows, slices, nW, c->line.p, c->lnw.p};
         il.cand = local ? c->candTri.p : nullptr;
         il.K = K;
         auto launchImportanceRows = [&](uint32_t nLaunchRows) {
-            launchImportance(cp->importanceLayers, il, c->layers, c->T, nLaunchRows, c->stream, true);
+            launchImportance(il, c->layers, c->T, c->Np, nLaunchRows, c->stream);
         };
         if (la) {
             pv.firstSample = firstSample;
@@ -3668,9 +3546,10 @@ hase_status hase_importance_weights(hase_context* c, uint32_t firstSample, uint3
     HASE_CUDA(q.ensure(size_t(count) * nW));
     HASE_CUDA(off.ensure(size_t(count) * (nW + 1)));
     HASE_CUDA(Q.ensure(count));
-    ImportanceLaunch il{c->view(), firstSample, slices, nW, float(meanA), float(meanB), lnw.p};
+    HASE_TRY(buildLineTable(c, meanA, meanB, slices, c->stream));
+    ImportanceLaunch il{c->view(), firstSample, count, slices, nW, c->line.p, lnw.p};
     localFields(c, il);
-    HASE_CUDA(launchImportance(0, il, c->layers, c->T, count, c->stream));
+    HASE_CUDA(launchImportance(il, c->layers, c->T, c->Np, count, c->stream));
     MapLaunch ml{lnw.p, 1, 1, nullptr, nW, 1u, nullptr, firstSample, 0u, 0u, 0u, w.p, q.p, Q.p, off.p};
     mapKernel<<<count, kMapBlock, 0, c->stream>>>(ml);
     HASE_CUDA(cudaGetLastError());
@@ -3727,10 +3606,11 @@ hase_status hase_importance_crossings(hase_context* c, uint32_t firstSample, uin
     HASE_CUDA(lnw.ensure(size_t(count) * nW));
     HASE_CUDA(n.ensure(1));
     HASE_CUDA(cudaMemsetAsync(n.p, 0, sizeof(unsigned long long), c->stream));
-    ImportanceLaunch il{c->view(), firstSample, slices, nW, 0.0f, 0.0f, lnw.p};
+    HASE_TRY(buildLineTable(c, 0.0, 0.0, slices, c->stream));
+    ImportanceLaunch il{c->view(), firstSample, count, slices, nW, c->line.p, lnw.p};
     localFields(c, il);
     il.crossings = n.p;
-    HASE_CUDA(launchImportance(0, il, c->layers, c->T, count, c->stream, false, true));
+    HASE_CUDA(launchImportance(il, c->layers, c->T, c->Np, count, c->stream, true));
     unsigned long long h = 0;
     HASE_CUDA(cudaMemcpyAsync(&h, n.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     HASE_CUDA(cudaStreamSynchronize(c->stream));
@@ -3833,7 +3713,16 @@ hase_status hase_mesh_tables(const hase_mesh_desc* d, float* tri, float* walk) {
     if (st != HASE_OK) return st;
     const size_t bytes = ht.tri.size() * sizeof(float4);
     if (tri) std::memcpy(tri, ht.tri.data(), bytes);
-    if (walk) std::memcpy(walk, ht.walk.data(), bytes);
+    if (walk) {  // the records with NaN normals on boundary edges
+        std::memcpy(walk, ht.tri.data(), bytes);
+        for (uint32_t t = 0; t < d->numberOfTriangles; ++t)
+            for (int e = 0; e < 3; ++e) {
+                float* r = walk + 12 * size_t(t);
+                int32_t nb;
+                std::memcpy(&nb, r + 9 + e, sizeof(nb));
+                if (nb < 0) r[3 * e] = r[3 * e + 1] = std::numeric_limits<float>::quiet_NaN();
+            }
+    }
     return HASE_OK;
 }
 
@@ -4270,6 +4159,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                               b->stream));
     HASE_CUDA(cudaMemcpyAsync(b->inst.p, views.data(), count * sizeof(InstanceView), cudaMemcpyHostToDevice,
                               b->stream));
+    uint32_t tableLaunches = 0;
     // learned proposal: one feature view per medium (coarse gain grid on the medium's context)
     std::vector<ProposalView> pviews;
     uint32_t proposalGrid = 0;
@@ -4295,6 +4185,14 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     // the views' gain grids are built on each context's own stream: finished
     // before the batch's stream reads them
     for (uint32_t i = 0; i < count; ++i) HASE_CUDA(cudaStreamSynchronize(media[i].c->stream));
+
+    // the importance lines' tables (on the batch's stream: every medium of a
+    // context has the same spectrum, so a context listed twice gets the same table)
+    for (uint32_t i = 0; i < count; ++i)
+        if (net ? fallbackVariance > 0.0f : !media[i].c->gridProposal) {
+            HASE_TRY(buildLineTable(media[i].c, media[i].meanA, media[i].meanB, slices, b->stream));
+            ++tableLaunches;
+        }
 
     // rows of every medium, cut into workspace chunks
     struct Chunk {
@@ -4363,6 +4261,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     }
 
     hase_batch_stats st{};
+    st.kernelLaunches = tableLaunches;
     st.rows = uint32_t(all.size());
     st.chunks = uint32_t(chunks.size());
     std::vector<uint32_t> unconvergedOf(count, 0), passesOf(count, 0);
@@ -4394,9 +4293,9 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                 const BatchMedium& md = media[i];
                 const hase_context* c = md.c;
                 const uint32_t segRows = uint32_t(e - r);
-                ImportanceLaunch il{views[i].m, all[r].sample, slices, md.nW, float(md.meanA), float(md.meanB),
+                ImportanceLaunch il{views[i].m, all[r].sample, segRows, slices, md.nW, c->line.p,
                                     b->lnw.p + all[r].w, nullptr, flag, uint32_t(r - ch.r0)};
-                HASE_CUDA(launchImportance(cp->importanceLayers, il, c->layers, c->T, segRows, b->stream));
+                HASE_CUDA(launchImportance(il, c->layers, c->T, c->Np, segRows, b->stream));
                 ++kernels;
                 return HASE_OK;
             };

@@ -69,8 +69,7 @@ __device__ __forceinline__ float unit24(uint32_t k24) { return (float(k24) + 0.5
 //   g0 = (ax, ay, bx-ax, by-ay), g1 = (cx-ax, cy-ay, area, 0); centroid separate.
 struct MeshView {
     const float4* tri;       // [T][3]
-    const float4* walk;      // [T][3]: tri with NaN normals on mesh-boundary edges (the importance walks' records)
-    const float4* win;       // [T][4]: the ray walk's edge windows (kWindowSlot)
+    const float4* win;       // [T][4]: the walks' edge windows (windowSlot)
     const float4* geo;       // [T][2]
     const int4* verts;       // [T] point ids of the triangle's vertices (w unused)
     const float2* centroid;  // [T]
@@ -79,11 +78,6 @@ struct MeshView {
     const float* srcBeta;    // [P] beta (source weight)
     const float2* points;    // [Np]
     const float* reflect;    // [T][2] or nullptr
-    // importance walks: per sample level, the slices x layers lines of a
-    // triangle ordered by their layer distance to the image level (without,
-    // with reflections), so that lines with similar numbers of level planes
-    // share a lane slot of the line teams
-    const uint16_t* lineOrder[2];
     uint32_t T, layers, P, Np;
     uint32_t divTm, divTs;   // floor(p / T) = (p * divTm) >> divTs for p < 2^31 (invariantDivisor)
     uint32_t divNpm, divNps; // the same for division by Np
@@ -93,7 +87,7 @@ struct MeshView {
     float tirCos2[2];        // total internal reflection when uz^2 <= tirCos2[surface]
 };
 
-// The ray walk's edge windows.  An edge is one float4 (nx, ny, c, code), a
+// The walks' edge windows.  An edge is one float4 (nx, ny, c, code), a
 // triangle holds its edges in the four slots e0 e1 e2 e0, and a window is the
 // pair of slots a ray that entered through the third edge can leave by:
 // entered through e0: slots 1, 2; e1: slots 2, 3; e2: slots 0, 1.  code is the
@@ -441,14 +435,5 @@ __device__ __forceinline__ bool nearFieldStart(const MeshView& m, uint32_t t, in
     alphaL = alpha * L;
     return true;
 }
-
-struct GlobalLoader {
-    const float4* tri;
-    __device__ __forceinline__ void operator()(uint32_t t, float4& a, float4& b, float4& c) const {
-        a = __ldg(tri + 3 * t);
-        b = __ldg(tri + 3 * t + 1);
-        c = __ldg(tri + 3 * t + 2);
-    }
-};
 
 }  // namespace hase

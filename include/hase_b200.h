@@ -106,9 +106,9 @@ typedef struct {
     uint64_t workspaceBytes;            /* 0 = default device workspace budget */
     uint32_t rayKernelVariant;          /* launch shape of the ray kernel, 0 = default; see
                                            hase_ray_kernel_variant_name (chosen by the autotuner) */
-    uint32_t importanceLayers;          /* importance kernel: 0 = line teams (a team of lanes per (sample,
-                                           triangle) shares the 2-D walk); 2, 4, 8 = that many prism layers
-                                           per thread; the same weights either way */
+    uint32_t importanceLayers;          /* 0, 2, 4 or 8: once the prism layers per thread of the importance
+                                           kernel; the library now chooses for every value (line teams),
+                                           the weights are the same */
 } hase_compute_desc;
 
 /* Caller-allocated host arrays of (maxSample - minSample + 1) entries; any
@@ -209,8 +209,9 @@ hase_status hase_importance_crossings(hase_context* ctx, uint32_t firstSample, u
  * unit normal and line constant (nx, ny, c) of its three edges followed by
  * the three neighbour codes as int bits (neighbour << 2 | the edge's index in
  * the neighbour, -1 at the mesh boundary), edge e joining the triangle's
- * points e and e + 1.  `tri` receives the records as given, `walk` the walks'
- * copy with NaN normals on the boundary edges; either may be NULL. */
+ * points e and e + 1 (the walks hold the same edges as two-edge windows).  `tri`
+ * receives the records, `walk` a copy with NaN normals on the boundary edges;
+ * either may be NULL. */
 hase_status hase_mesh_tables(const hase_mesh_desc* mesh, float* tri, float* walk);
 
 /* Ray->prism map of `rows` weight rows of length n: q[row][n] (quantised
