@@ -66,7 +66,7 @@ constexpr uint32_t kRayBlock = 256;
 constexpr int kRayMinBlocks = 5;
 constexpr int kRefill = 8;  // idle lanes that trigger a batched refill
 constexpr uint32_t kMaxItems = 1024;  // work items per sample and pass
-constexpr uint32_t kMinItemRays = 1024;
+constexpr uint32_t kMinItemRays = 64, kMaxAutoItemRays = 1024;  // rays per work item of the default launch
 constexpr uint32_t kMapBlock = 1024;
 #ifndef HASE_WALK_COLUMNS
 #define HASE_WALK_COLUMNS 32
@@ -721,6 +721,22 @@ __device__ __forceinline__ uint32_t warpEntries(const uint32_t* off, uint32_t b0
     return b;
 }
 
+// Elements of a[0, n) (non-decreasing) that do not exceed x, by the whole warp:
+// 32 probes a round, so 4 dependent loads for a row of half a million entries
+// where a binary search takes 19.
+__device__ __forceinline__ uint32_t warpUpperBound(const uint32_t* a, uint32_t n, uint32_t x) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0;
+    while (n > 0) {
+        const uint32_t step = (n + 31u) / 32u, i = (lane + 1u) * step - 1u;
+        const bool in = i < n && __ldg(a + lo + i) <= x;
+        const uint32_t below = uint32_t(__popc(__ballot_sync(0xffffffffu, in))) * step;
+        lo += below;
+        n = min(step - 1u, n - below);
+    }
+    return lo;
+}
+
 // log2 of the entries between warpEntries' offsets for `rays` rays in `entries` entries.
 __device__ __forceinline__ uint32_t entryShift(uint32_t entries, uint32_t rays) {
     return entries <= rays ? 0u : 31u - uint32_t(__clz(int(2u * entries / rays)));
@@ -950,13 +966,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
         // prisms holding the item's mapped rays [r0, rn1): [pb, pb + count - 1)
         // (the local proposal maps its near rays [0, Mnear) only)
         const uint32_t rn1 = LOCAL ? min(r1, L.Mnear) : r1;
-        uint32_t bound = 0;
+        uint32_t pb = 0, count = 0;
         if (r0 < rn1) {
-            if (lane == 0) bound = upperBound(off, nW + 1, r0) - 1u;
-            if (lane == 1) bound = upperBound(off, nW + 1, rn1 - 1u) - 1u;
+            pb = warpUpperBound(off, nW + 1, r0) - 1u;
+            count = warpUpperBound(off + pb, nW + 1 - pb, rn1 - 1u) + 1u;
         }
-        const uint32_t pb = __shfl_sync(0xffffffffu, bound, 0);
-        const uint32_t count = r0 < rn1 ? __shfl_sync(0xffffffffu, bound, 1) - pb + 2u : 0u;
 
         double sum = 0.0, sum2 = 0.0;
         uint32_t dropped = 0, crossings = 0;
@@ -2208,6 +2222,18 @@ hase_status uploadBeta(hase_context* c, const double* betaVolume) {
     return HASE_OK;
 }
 
+// Rays per work item of a pass of M rays per sample: 32 x raysPerThread, or
+// about 256 items a row (64 to 1024 rays each; 1024 is the measured best where
+// the rows alone fill the device many times over, by 2 % against 384, but it
+// left 50 items for 50,000 rays (ray kernel 127 us, 23 us with 64) and a last
+// wave of whole items for 256 rows x 1e5 rays (6.2 ms, 5.4 with 384)).  It
+// depends on M alone, so that a sample's sums do not depend on the other
+// samples of the call.
+uint32_t itemRaysOf(uint32_t M, uint32_t raysPerThread) {
+    const uint32_t automatic = std::min(kMaxAutoItemRays, std::max(kMinItemRays, (M / 256u + 31u) & ~31u));
+    return std::max<uint32_t>(raysPerThread ? 32u * raysPerThread : automatic, (M + kMaxItems - 1) / kMaxItems);
+}
+
 uint32_t adaptiveTarget(uint32_t minRays, uint32_t maxRays, uint32_t steps, uint32_t k) {
     // include/core/types.hpp:333-354: geometric growth minRays -> maxRays in `steps` increases.
     if (maxRays <= minRays || steps == 0) return minRays;
@@ -2913,8 +2939,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
                          nullptr, c->q.p, c->Q.p, c->offsets.p};
             mapKernel<<<nActive, kMapBlock, 0, c->stream>>>(ml);
             HASE_CUDA(cudaGetLastError());
-            const uint32_t itemRays = std::max<uint32_t>(cp->raysPerThread ? 32u * cp->raysPerThread : kMinItemRays,
-                                                         (M + kMaxItems - 1) / kMaxItems);
+            const uint32_t itemRays = itemRaysOf(M, cp->raysPerThread);
             const uint32_t items = (M + itemRays - 1) / itemRays;
             HASE_CUDA(cudaMemsetAsync(c->itemCounter.p, 0, sizeof(unsigned int), c->stream));
             HASE_CUDA(cudaEventRecord(c->ev[2], c->stream));
@@ -3917,7 +3942,7 @@ hase_status hase_estimate_sample_noalloc(hase_context* c, uint32_t sample, const
                  nullptr, q, Q, offsets};
     mapKernel<<<1, kMapBlock, 0, c->stream>>>(ml);
     HASE_CUDA(cudaGetLastError());
-    const uint32_t itemRays = std::max<uint32_t>(kMinItemRays, (rays + kMaxItems - 1) / kMaxItems);
+    const uint32_t itemRays = itemRaysOf(rays, 0u);
     const uint32_t items = (rays + itemRays - 1) / itemRays;
     const double C = c->nTot / (4.0 * kPi * c->tau);
     RayLaunch rl{mv, active, 1u, sample, 0u, rays, uint32_t(nW), itemRays, items, itemCounter, q, Q, offsets,
@@ -4130,8 +4155,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
         const bool last = target >= maxRays || pass >= cp->adaptiveSteps;
         Pass ps;
         ps.M = target - prev;
-        ps.itemRays = std::max<uint32_t>(cp->raysPerThread ? 32u * cp->raysPerThread : kMinItemRays,
-                                         (ps.M + kMaxItems - 1) / kMaxItems);
+        ps.itemRays = itemRaysOf(ps.M, cp->raysPerThread);
         ps.items = (ps.M + ps.itemRays - 1) / ps.itemRays;
         ps.last = last;
         passes.push_back(ps);
