@@ -425,6 +425,7 @@ struct MapLaunch {
     const RowInfo* rows;        // batched media: ragged rows (nW, workspace offset, sample, seed per row)
     const unsigned int* count;  // batched media: rows of rowList to map (device), blocks stride over them
     const uint8_t* rowFlag;     // batched media: only rows with rowFlag[row] set are mapped (or null)
+    unsigned int* zero[2];      // counters of the pass's ray and finalise launches, zeroed here (or null)
 };
 
 // Each warp owns one contiguous segment of the row (a multiple of 32 entries
@@ -561,6 +562,7 @@ __device__ void mapRow(const MapLaunch& L, uint32_t row) {
 // device-held number of rows.
 __global__ void __launch_bounds__(kMapBlock, 2) mapKernel(MapLaunch L) {
     const uint32_t n = L.count ? *L.count : gridDim.x;
+    if (blockIdx.x == 0 && threadIdx.x < 2 && L.zero[threadIdx.x]) *L.zero[threadIdx.x] = 0u;
     for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
         const uint32_t row = L.rowList ? L.rowList[i] : i;
         if (L.rowFlag && !L.rowFlag[row]) continue;  // uniform over the block
@@ -1182,9 +1184,40 @@ __device__ void finalizeRow(const FinalizeLaunch& L, uint32_t row, int lane) {
     }
 }
 
-__global__ void iotaKernel(uint32_t* a, uint32_t n) {
+// The per-row accumulators and results of n rows in one block: sum, sum2, then
+// (the part that goes to the host, in one copy) rse, crossings, rays, dropped, phi.
+struct RowView {
+    double *sum, *sum2, *mse;
+    unsigned long long* cross;
+    uint32_t *total, *drop;
+    float* phi;
+};
+constexpr size_t kRowSumBytes = 16, kRowResultBytes = 28;
+RowView rowView(unsigned char* sums, unsigned char* results, size_t n) {
+    RowView v;
+    v.sum = reinterpret_cast<double*>(sums);
+    v.sum2 = sums ? v.sum + n : nullptr;
+    v.mse = reinterpret_cast<double*>(results);
+    v.cross = reinterpret_cast<unsigned long long*>(v.mse + n);
+    v.total = reinterpret_cast<uint32_t*>(v.cross + n);
+    v.drop = v.total + n;
+    v.phi = reinterpret_cast<float*>(v.drop + n);
+    return v;
+}
+
+// The rows of a solve before its first pass: every row active, nothing summed,
+// the counters zero (counts[0] = n in a batched solve).
+__global__ void initRowsKernel(RowView v, uint32_t n, uint32_t* active, unsigned int* counts, uint32_t nCounts,
+                               int batched) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = i;
+    if (i < nCounts) counts[i] = batched && i == 0 ? n : 0u;
+    if (i >= n) return;
+    active[i] = i;
+    v.sum[i] = 0.0;
+    v.sum2[i] = 0.0;
+    v.total[i] = 0u;
+    v.drop[i] = 0u;
+    v.cross[i] = 0ull;
 }
 
 // Batched learned solve, after the first pass: the still-active rows whose
@@ -1217,13 +1250,6 @@ __global__ void resetFlaggedKernel(const uint32_t* active, const unsigned int* c
         drop[row] = 0u;
         cross[row] = 0ull;
     }
-}
-
-// iota plus the device-held row count of a batched solve's first pass.
-__global__ void iotaCountKernel(uint32_t* a, uint32_t n, unsigned int* count) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = i;
-    if (i == 0) *count = n;
 }
 
 // ------------------------------------------------------ diagnostics ----
@@ -2147,13 +2173,13 @@ struct hase_context {
     DevBuf<float> gTab;  // g of every prism for the spectrally averaged (A, B) of the last solve
     // workspace
     DevBuf<float> lnw;
-    DevBuf<uint32_t> q, offsets, activeA, activeB, counter, accTotal, accDrop, pDrop;
-    DevBuf<unsigned int> itemCounter;
+    DevBuf<uint32_t> q, offsets, activeA, activeB, pDrop;
+    DevBuf<unsigned char> rowState;  // RowView
+    DevBuf<unsigned int> counters;  // [0] rays' work items taken, [1] samples still above the threshold
     uint32_t persistentBlocks = 0;  // resident rayKernel blocks on the device
     uint32_t variantBlocks[3][16] = {};  // the same for every walk mode x launch shape of kRayVariants (at most 16)
-    DevBuf<unsigned long long> Q, accCross, pCross;
-    DevBuf<double> accSum, accSum2, pSum, pSum2, mse;
-    DevBuf<float> phi;
+    DevBuf<unsigned long long> Q, pCross;
+    DevBuf<double> pSum, pSum2;
     // host copies used by the learned proposal's features
     std::vector<float2> hCentroid, hPoints;
     std::vector<float> hArea, hGainBeta, hReflect;
@@ -2781,8 +2807,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     }
     HASE_CUDA(c->activeA.ensure(rows));
     HASE_CUDA(c->activeB.ensure(rows));
-    HASE_CUDA(c->counter.ensure(1));
-    HASE_CUDA(c->itemCounter.ensure(1));
+    HASE_CUDA(c->counters.ensure(2));
     if (!validImportanceLayers(cp->importanceLayers))
         return fail(HASE_INVALID_ARGUMENT, "importanceLayers must be 0, 2, 4 or 8");
     if (cp->rayKernelVariant >= kNumRayVariants)
@@ -2805,13 +2830,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
         HASE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
         c->persistentBlocks = uint32_t(std::max(1, perSM) * std::max(1, sms));
     }
-    HASE_CUDA(c->accSum.ensure(rows));
-    HASE_CUDA(c->accSum2.ensure(rows));
-    HASE_CUDA(c->accTotal.ensure(rows));
-    HASE_CUDA(c->accDrop.ensure(rows));
-    HASE_CUDA(c->accCross.ensure(rows));
-    HASE_CUDA(c->phi.ensure(rows));
-    HASE_CUDA(c->mse.ensure(rows));
+    HASE_CUDA(c->rowState.ensure(size_t(rows) * (kRowSumBytes + kRowResultBytes)));
     HASE_CUDA(c->pSum.ensure(size_t(rows) * kMaxItems));
     HASE_CUDA(c->pSum2.ensure(size_t(rows) * kMaxItems));
     HASE_CUDA(c->pDrop.ensure(size_t(rows) * kMaxItems));
@@ -2850,10 +2869,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     }
     const MeshView mv = c->view();
     const double C = c->nTot / (4.0 * kPi * c->tau);
-    std::vector<float> hPhi(rows);
-    std::vector<double> hMse(rows);
-    std::vector<uint32_t> hTotal(rows), hDrop(rows);
-    std::vector<unsigned long long> hCross(rows);
+    std::vector<unsigned char> hResults(size_t(rows) * kRowResultBytes);
     res->raysTraced = 0;
     res->crossings = 0;
     res->importanceMilliseconds = 0;
@@ -2911,14 +2927,10 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
         HASE_CUDA(cudaGetLastError());
         if (logOut) HASE_CUDA(cudaMemsetAsync(c->logBuf.p, 0, size_t(nRows) * nW * sizeof(float), c->stream));
         HASE_CUDA(cudaEventRecord(c->ev[1], c->stream));
-        HASE_CUDA(cudaMemsetAsync(c->accSum.p, 0, nRows * sizeof(double), c->stream));
-        HASE_CUDA(cudaMemsetAsync(c->accSum2.p, 0, nRows * sizeof(double), c->stream));
-        HASE_CUDA(cudaMemsetAsync(c->accTotal.p, 0, nRows * sizeof(uint32_t), c->stream));
-        HASE_CUDA(cudaMemsetAsync(c->accDrop.p, 0, nRows * sizeof(uint32_t), c->stream));
-        HASE_CUDA(cudaMemsetAsync(c->accCross.p, 0, nRows * sizeof(unsigned long long), c->stream));
-        iotaKernel<<<(nRows + 255) / 256, 256, 0, c->stream>>>(c->activeA.p, nRows);
+        const RowView rv{rowView(c->rowState.p, c->rowState.p + size_t(nRows) * kRowSumBytes, nRows)};
+        initRowsKernel<<<(nRows + 255) / 256, 256, 0, c->stream>>>(rv, nRows, c->activeA.p, c->counters.p, 2u, 0);
         HASE_CUDA(cudaGetLastError());
-        res->kernelLaunches += 2;  // importance + iota
+        res->kernelLaunches += 2;  // importance + row state
         uint32_t* cur = c->activeA.p;
         uint32_t* nxt = c->activeB.p;
         uint32_t nActive = nRows;
@@ -2937,13 +2949,14 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             const uint32_t Mnear = M - Mfar;
             MapLaunch ml{c->lnw.p, 1, pass == 0 ? 1 : 0, cur, nW, Mnear, nullptr, firstSample, pass, cp->rngSeed, 0u,
                          nullptr, c->q.p, c->Q.p, c->offsets.p};
+            ml.zero[0] = c->counters.p;
+            ml.zero[1] = c->counters.p + 1;
             mapKernel<<<nActive, kMapBlock, 0, c->stream>>>(ml);
             HASE_CUDA(cudaGetLastError());
             const uint32_t itemRays = itemRaysOf(M, cp->raysPerThread);
             const uint32_t items = (M + itemRays - 1) / itemRays;
-            HASE_CUDA(cudaMemsetAsync(c->itemCounter.p, 0, sizeof(unsigned int), c->stream));
             HASE_CUDA(cudaEventRecord(c->ev[2], c->stream));
-            RayLaunch rl{mv, cur, nActive, firstSample, pass, M, nW, itemRays, items, c->itemCounter.p, c->q.p,
+            RayLaunch rl{mv, cur, nActive, firstSample, pass, M, nW, itemRays, items, c->counters.p, c->q.p,
                          c->Q.p, c->offsets.p, cp->rngSeed, 0u, c->spec.p, nLambda, ex->nearFieldSampling, C, c->pSum.p, c->pSum2.p,
                          c->pDrop.p, c->pCross.p, logOut ? c->logBuf.p : nullptr};
             if (local) {
@@ -2962,30 +2975,29 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             const RayVariant logVariant{rayKernel<kRayBlock, kRefill, kRayMinBlocks, true>, int(kRayBlock), "log"};
             const RayVariant localLog{rayKernel<kRayBlock, kRefill, kRayMinBlocks, true, false, kWalkColumns, kWalkBeta, true>,
                                       int(kRayBlock), "local log"};
-            const RayVariant& rv = local ? (logOut ? localLog : kLocalVariant) : (logOut ? logVariant : kRayVariants[variant]);
+            const RayVariant& shape = local ? (logOut ? localLog : kLocalVariant) : (logOut ? logVariant : kRayVariants[variant]);
             const uint64_t totalItems = uint64_t(nActive) * items;
-            void (*const kern)(RayLaunch) = walk == kWalkTable ? rv.mono : (walk == kWalkBetaNoClad ? rv.noClad : rv.kernel);
+            void (*const kern)(RayLaunch) = walk == kWalkTable ? shape.mono : (walk == kWalkBetaNoClad ? shape.noClad : shape.kernel);
             uint32_t resident = c->variantBlocks[walk][variant];
             if (local) {  // occupancy of the local kernel itself
                 int perSM = 0, sms = 0;
-                HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, rv.block, 0));
+                HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, shape.block, 0));
                 HASE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
                 resident = uint32_t(std::max(1, perSM) * std::max(1, sms));
             }
-            const uint32_t grid = uint32_t(std::min<uint64_t>(totalItems / (rv.block / 32) + 1, uint64_t(resident)));
+            const uint32_t grid = uint32_t(std::min<uint64_t>(totalItems / (shape.block / 32) + 1, uint64_t(resident)));
             void* rayArgs[] = {&rl};
-            HASE_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(rv.block), rayArgs, 0,
+            HASE_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(shape.block), rayArgs, 0,
                                        c->stream));
             HASE_CUDA(cudaEventRecord(c->ev[3], c->stream));
-            HASE_CUDA(cudaMemsetAsync(c->counter.p, 0, sizeof(uint32_t), c->stream));
             FinalizeLaunch fl{cur, nActive, items, M, lastPass ? 1 : 0, ex->mseThreshold, c->pSum.p, c->pSum2.p,
-                              c->pDrop.p, c->pCross.p, c->accSum.p, c->accSum2.p, c->accTotal.p, c->accDrop.p,
-                              c->accCross.p, c->phi.p, c->mse.p, nxt, c->counter.p};
+                              c->pDrop.p, c->pCross.p, rv.sum, rv.sum2, rv.total, rv.drop, rv.cross, rv.phi, rv.mse,
+                              nxt, c->counters.p + 1};
             finalizeKernel<<<(nActive * 32 + 127) / 128, 128, 0, c->stream>>>(fl);
             HASE_CUDA(cudaGetLastError());
             res->kernelLaunches += 3;  // map + rays + finalize
             uint32_t next = 0;
-            HASE_CUDA(cudaMemcpyAsync(&next, c->counter.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+            HASE_CUDA(cudaMemcpyAsync(&next, c->counters.p + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
             HASE_CUDA(cudaStreamSynchronize(c->stream));
             float ms = 0;
             if (pass == 0) {
@@ -3009,8 +3021,8 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
                 hRse.resize(nRows);
                 hTot.resize(nRows);
                 HASE_CUDA(cudaMemcpyAsync(hList.data(), nxt, next * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-                HASE_CUDA(cudaMemcpyAsync(hRse.data(), c->mse.p, nRows * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-                HASE_CUDA(cudaMemcpyAsync(hTot.data(), c->accTotal.p, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                HASE_CUDA(cudaMemcpyAsync(hRse.data(), rv.mse, nRows * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+                HASE_CUDA(cudaMemcpyAsync(hTot.data(), rv.total, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                           c->stream));
                 HASE_CUDA(cudaStreamSynchronize(c->stream));
                 std::vector<uint32_t> fb;
@@ -3032,9 +3044,8 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
                     MapLaunch rq{c->lnw.p, 1, 1, c->rowList.p, nW, 1u, nullptr, firstSample, 0u, cp->rngSeed, 0u,
                                  nullptr, c->q.p, c->Q.p, c->offsets.p};
                     mapKernel<<<nf, kMapBlock, 0, c->stream>>>(rq);
-                    resetRowsKernel<<<(nf + 255) / 256, 256, 0, c->stream>>>(c->rowList.p, nf, c->accSum.p,
-                                                                             c->accSum2.p, c->accTotal.p,
-                                                                             c->accDrop.p, c->accCross.p);
+                    resetRowsKernel<<<(nf + 255) / 256, 256, 0, c->stream>>>(c->rowList.p, nf, rv.sum, rv.sum2,
+                                                                             rv.total, rv.drop, rv.cross);
                     HASE_CUDA(cudaGetLastError());
                     res->kernelLaunches += 3;
                     HASE_CUDA(cudaStreamSynchronize(c->stream));
@@ -3048,11 +3059,8 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             nActive = next;
         }
         HASE_CUDA(cudaEventRecord(c->ev[3], c->stream));
-        HASE_CUDA(cudaMemcpyAsync(hPhi.data(), c->phi.p, nRows * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-        HASE_CUDA(cudaMemcpyAsync(hMse.data(), c->mse.p, nRows * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        HASE_CUDA(cudaMemcpyAsync(hTotal.data(), c->accTotal.p, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-        HASE_CUDA(cudaMemcpyAsync(hDrop.data(), c->accDrop.p, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-        HASE_CUDA(cudaMemcpyAsync(hCross.data(), c->accCross.p, nRows * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+        HASE_CUDA(cudaMemcpyAsync(hResults.data(), c->rowState.p + size_t(nRows) * kRowSumBytes,
+                                  size_t(nRows) * kRowResultBytes, cudaMemcpyDeviceToHost, c->stream));
         if (logOut)
             HASE_CUDA(cudaMemcpyAsync(logOut + size_t(b0) * nW, c->logBuf.p, size_t(nRows) * nW * sizeof(float),
                                       cudaMemcpyDeviceToHost, c->stream));
@@ -3060,21 +3068,22 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
         float total = 0;
         HASE_CUDA(cudaEventElapsedTime(&total, c->ev[0], c->ev[3]));
         res->totalMilliseconds += total;
+        const RowView h = rowView(nullptr, hResults.data(), nRows);
         for (uint32_t i = 0; i < nRows; ++i) {
             const uint32_t o = b0 + i, s = firstSample + i;
-            if (res->phiAse) res->phiAse[o] = hPhi[i];
-            if (res->relativeStandardError) res->relativeStandardError[o] = hMse[i];
-            if (res->standardError) res->standardError[o] = hMse[i] * double(hPhi[i]);
-            if (res->totalRays) res->totalRays[o] = hTotal[i];
-            if (res->droppedRays) res->droppedRays[o] = hDrop[i];
+            if (res->phiAse) res->phiAse[o] = h.phi[i];
+            if (res->relativeStandardError) res->relativeStandardError[o] = h.mse[i];
+            if (res->standardError) res->standardError[o] = h.mse[i] * double(h.phi[i]);
+            if (res->totalRays) res->totalRays[o] = h.total[i];
+            if (res->droppedRays) res->droppedRays[o] = h.drop[i];
             if (res->dndtAse) {
                 const double sA = nLambda == 1 ? c->sigmaA[0] : maxSA, sE = nLambda == 1 ? c->sigmaE[0] : maxSE;
                 const double bc = c->betaCells.empty() ? 0.0 : c->betaCells[s];
-                res->dndtAse[o] = (bc * (sE + sA) - sA) * double(hPhi[i]);
+                res->dndtAse[o] = (bc * (sE + sA) - sA) * double(h.phi[i]);
             }
-            res->raysTraced += hTotal[i];
-            res->crossings += hCross[i];
-            droppedTotal += hDrop[i];
+            res->raysTraced += h.total[i];
+            res->crossings += h.cross[i];
+            droppedTotal += h.drop[i];
         }
     }
     if (droppedTotal) {
@@ -3974,12 +3983,13 @@ struct hase_batch {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::vector<cudaEvent_t> ev;  // timing events recorded inside the graphs
-    DevBuf<float> lnw, phi, prior;
+    DevBuf<float> lnw, prior;
+    DevBuf<unsigned char> rowState;  // RowView
     DevBuf<uint8_t> rowFlag;      // rows restarting with the importance weights (learned solve)
-    DevBuf<uint32_t> q, offsets, activeA, activeB, accTotal, accDrop, pDrop;
+    DevBuf<uint32_t> q, offsets, activeA, activeB, pDrop;
     DevBuf<unsigned int> counts;  // [0], [1]: active rows (alternating), [2]: item counter, [3 ..]: per pass
-    DevBuf<unsigned long long> Q, accCross, pCross;
-    DevBuf<double> accSum, accSum2, pSum, pSum2, mse;
+    DevBuf<unsigned long long> Q, pCross;
+    DevBuf<double> pSum, pSum2;
     DevBuf<float2> spec;
     DevBuf<InstanceView> inst;
     DevBuf<RowInfo> rows;
@@ -4266,13 +4276,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     HASE_CUDA(b->counts.ensure(4 + nPasses));
     const bool fallback = net && fallbackVariance > 0.0f && nPasses > 1;
     if (fallback) HASE_CUDA(b->rowFlag.ensure(maxRows));
-    HASE_CUDA(b->accSum.ensure(maxRows));
-    HASE_CUDA(b->accSum2.ensure(maxRows));
-    HASE_CUDA(b->accTotal.ensure(maxRows));
-    HASE_CUDA(b->accDrop.ensure(maxRows));
-    HASE_CUDA(b->accCross.ensure(maxRows));
-    HASE_CUDA(b->phi.ensure(maxRows));
-    HASE_CUDA(b->mse.ensure(maxRows));
+    HASE_CUDA(b->rowState.ensure(maxRows * (kRowSumBytes + kRowResultBytes)));
     HASE_CUDA(b->pSum.ensure(maxRows * kMaxItems));
     HASE_CUDA(b->pSum2.ensure(maxRows * kMaxItems));
     HASE_CUDA(b->pDrop.ensure(maxRows * kMaxItems));
@@ -4291,10 +4295,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     std::vector<uint32_t> unconvergedOf(count, 0), passesOf(count, 0);
     std::vector<uint64_t> raysOf(count, 0), crossOf(count, 0);
     uint64_t droppedTotal = 0;
-    std::vector<float> hPhi(maxRows);
-    std::vector<double> hMse(maxRows);
-    std::vector<uint32_t> hTotal(maxRows), hDrop(maxRows), hCounts(4 + nPasses);
-    std::vector<unsigned long long> hCross(maxRows);
+    std::vector<unsigned char> hResults(maxRows * kRowResultBytes);
+    std::vector<uint32_t> hCounts(4 + nPasses);
     const double thr = ex->mseThreshold;
 
     for (const Chunk& ch : chunks) {
@@ -4303,6 +4305,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
         HASE_CUDA(cudaMemcpyAsync(b->rows.p, all.data() + ch.r0, nRows * sizeof(RowInfo), cudaMemcpyHostToDevice,
                                   b->stream));
         HASE_CUDA(cudaStreamSynchronize(b->stream));
+        const RowView rw{rowView(b->rowState.p, b->rowState.p + size_t(nRows) * kRowSumBytes, nRows)};
         const auto tc0 = std::chrono::steady_clock::now();
         GraphOwner graph;
         uint32_t kernels = 0;
@@ -4362,13 +4365,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                 HASE_CUDA(cudaGetLastError());
             }
             HASE_CUDA(cudaEventRecordWithFlags(b->ev[1], b->stream, cudaEventRecordExternal));
-            HASE_CUDA(cudaMemsetAsync(b->accSum.p, 0, nRows * sizeof(double), b->stream));
-            HASE_CUDA(cudaMemsetAsync(b->accSum2.p, 0, nRows * sizeof(double), b->stream));
-            HASE_CUDA(cudaMemsetAsync(b->accTotal.p, 0, nRows * sizeof(uint32_t), b->stream));
-            HASE_CUDA(cudaMemsetAsync(b->accDrop.p, 0, nRows * sizeof(uint32_t), b->stream));
-            HASE_CUDA(cudaMemsetAsync(b->accCross.p, 0, nRows * sizeof(unsigned long long), b->stream));
-            HASE_CUDA(cudaMemsetAsync(b->counts.p, 0, (4 + nPasses) * sizeof(unsigned int), b->stream));
-            iotaCountKernel<<<(nRows + 255) / 256, 256, 0, b->stream>>>(b->activeA.p, nRows, b->counts.p);
+            initRowsKernel<<<(std::max(nRows, 4 + nPasses) + 255) / 256, 256, 0, b->stream>>>(
+                rw, nRows, b->activeA.p, b->counts.p, 4 + nPasses, 1);
             HASE_CUDA(cudaGetLastError());
             ++kernels;
             uint32_t* cur = b->activeA.p;
@@ -4384,9 +4382,10 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                                           b->stream));
                 MapLaunch ml{b->lnw.p, 1, k == 0 ? 1 : 0, cur, 0u, ps.M, nullptr, 0u, k, 0u, 0u, nullptr, b->q.p,
                              b->Q.p, b->offsets.p, b->rows.p, cntCur};
+                ml.zero[0] = itemCounter;
+                ml.zero[1] = cntNxt;
                 mapKernel<<<mapGrid, kMapBlock, 0, b->stream>>>(ml);
                 HASE_CUDA(cudaGetLastError());
-                HASE_CUDA(cudaMemsetAsync(itemCounter, 0, sizeof(unsigned int), b->stream));
                 HASE_CUDA(cudaEventRecordWithFlags(b->ev[3 + 2 * k], b->stream, cudaEventRecordExternal));
                 RayLaunch rl{};
                 rl.active = cur;
@@ -4412,10 +4411,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                 HASE_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(noClad ? rv.noClad : rv.kernel), dim3(grid),
                                            dim3(rv.block), rayArgs, 0, b->stream));
                 HASE_CUDA(cudaEventRecordWithFlags(b->ev[4 + 2 * k], b->stream, cudaEventRecordExternal));
-                HASE_CUDA(cudaMemsetAsync(cntNxt, 0, sizeof(unsigned int), b->stream));
                 FinalizeLaunch fl{cur, 0u, ps.items, ps.M, ps.last ? 1 : 0, thr, b->pSum.p, b->pSum2.p, b->pDrop.p,
-                                  b->pCross.p, b->accSum.p, b->accSum2.p, b->accTotal.p, b->accDrop.p, b->accCross.p,
-                                  b->phi.p, b->mse.p, nxt, cntNxt, cntCur};
+                                  b->pCross.p, rw.sum, rw.sum2, rw.total, rw.drop, rw.cross, rw.phi, rw.mse, nxt, cntNxt, cntCur};
                 finalizeKernel<<<finGrid, 128, 0, b->stream>>>(fl);
                 HASE_CUDA(cudaGetLastError());
                 kernels += 3;
@@ -4427,7 +4424,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                     // importance weights (as hase_calc_phi_ase_learned does, on the device)
                     const uint32_t g = std::min<uint32_t>((nRows + 255) / 256, uint32_t(8 * b->sms));
                     HASE_CUDA(cudaMemsetAsync(b->rowFlag.p, 0, nRows, b->stream));
-                    fallbackMarkKernel<<<g, 256, 0, b->stream>>>(cur, cntCur, b->accTotal.p, b->mse.p,
+                    fallbackMarkKernel<<<g, 256, 0, b->stream>>>(cur, cntCur, rw.total, rw.mse,
                                                                  double(fallbackVariance), b->rowFlag.p,
                                                                  b->counts.p + 3 + nPasses);
                     HASE_CUDA(cudaGetLastError());
@@ -4435,8 +4432,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                     MapLaunch rq{b->lnw.p, 1, 1, cur, 0u, 1u, nullptr, 0u, 0u, 0u, 0u, nullptr, b->q.p, b->Q.p,
                                  b->offsets.p, b->rows.p, cntCur, b->rowFlag.p};
                     mapKernel<<<mapGrid, kMapBlock, 0, b->stream>>>(rq);
-                    resetFlaggedKernel<<<g, 256, 0, b->stream>>>(cur, cntCur, b->rowFlag.p, b->accSum.p, b->accSum2.p,
-                                                                 b->accTotal.p, b->accDrop.p, b->accCross.p);
+                    resetFlaggedKernel<<<g, 256, 0, b->stream>>>(cur, cntCur, b->rowFlag.p, rw.sum, rw.sum2, rw.total,
+                                                                 rw.drop, rw.cross);
                     HASE_CUDA(cudaGetLastError());
                     kernels += 3;
                 }
@@ -4455,14 +4452,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
         st.captureMilliseconds +=
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tc0).count();
         HASE_CUDA(cudaGraphLaunch(graph.x, b->stream));
-        HASE_CUDA(cudaMemcpyAsync(hPhi.data(), b->phi.p, nRows * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-        HASE_CUDA(cudaMemcpyAsync(hMse.data(), b->mse.p, nRows * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-        HASE_CUDA(cudaMemcpyAsync(hTotal.data(), b->accTotal.p, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                  b->stream));
-        HASE_CUDA(cudaMemcpyAsync(hDrop.data(), b->accDrop.p, nRows * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                  b->stream));
-        HASE_CUDA(cudaMemcpyAsync(hCross.data(), b->accCross.p, nRows * sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, b->stream));
+        HASE_CUDA(cudaMemcpyAsync(hResults.data(), b->rowState.p + size_t(nRows) * kRowSumBytes,
+                                  size_t(nRows) * kRowResultBytes, cudaMemcpyDeviceToHost, b->stream));
         HASE_CUDA(cudaMemcpyAsync(hCounts.data(), b->counts.p, (4 + nPasses) * sizeof(unsigned int),
                                   cudaMemcpyDeviceToHost, b->stream));
         HASE_CUDA(cudaStreamSynchronize(b->stream));
@@ -4481,32 +4472,33 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
         st.kernelLaunches += kernels;
         st.graphNodes += uint32_t(nodes);
         // scatter the chunk's rows into the media's results
+        const RowView h = rowView(nullptr, hResults.data(), nRows);
         for (uint32_t j = 0; j < nRows; ++j) {
             const RowInfo& ri = all[ch.r0 + j];
             const BatchMedium& md = media[ri.inst];
             hase_result* res = in[ri.inst].result;
             const uint32_t o = ri.sample - md.first;
-            if (res->phiAse) res->phiAse[o] = hPhi[j];
-            if (res->relativeStandardError) res->relativeStandardError[o] = hMse[j];
-            if (res->standardError) res->standardError[o] = hMse[j] * double(hPhi[j]);
-            if (res->totalRays) res->totalRays[o] = hTotal[j];
-            if (res->droppedRays) res->droppedRays[o] = hDrop[j];
+            if (res->phiAse) res->phiAse[o] = h.phi[j];
+            if (res->relativeStandardError) res->relativeStandardError[o] = h.mse[j];
+            if (res->standardError) res->standardError[o] = h.mse[j] * double(h.phi[j]);
+            if (res->totalRays) res->totalRays[o] = h.total[j];
+            if (res->droppedRays) res->droppedRays[o] = h.drop[j];
             if (res->dndtAse) {
                 const double bc = md.c->betaCells.empty() ? 0.0 : md.c->betaCells[ri.sample];
-                res->dndtAse[o] = (bc * (md.sE + md.sA) - md.sA) * double(hPhi[j]);
+                res->dndtAse[o] = (bc * (md.sE + md.sA) - md.sA) * double(h.phi[j]);
             }
-            if (!(hMse[j] <= thr)) ++unconvergedOf[ri.inst];
+            if (!(h.mse[j] <= thr)) ++unconvergedOf[ri.inst];
             uint32_t np = 0;
-            for (uint32_t k = 0, cum = 0; k < nPasses && cum < hTotal[j]; ++k) {
+            for (uint32_t k = 0, cum = 0; k < nPasses && cum < h.total[j]; ++k) {
                 cum += passes[k].M;
                 np = k + 1;
             }
             passesOf[ri.inst] = std::max(passesOf[ri.inst], np);
-            raysOf[ri.inst] += hTotal[j];
-            crossOf[ri.inst] += hCross[j];
-            droppedTotal += hDrop[j];
-            st.raysTraced += hTotal[j];
-            st.crossings += hCross[j];
+            raysOf[ri.inst] += h.total[j];
+            crossOf[ri.inst] += h.cross[j];
+            droppedTotal += h.drop[j];
+            st.raysTraced += h.total[j];
+            st.crossings += h.cross[j];
         }
     }
     for (uint32_t i = 0; i < count; ++i) {
