@@ -592,18 +592,44 @@ __global__ void __launch_bounds__(256) fwdFinalizeKernel(const FinLaunch F) {
     if (!(isfinite(rse) && rse <= F.threshold)) atomicAdd(F.unconverged, 1u);
 }
 
-// Inclusive CDF of one batch's reservoir face weights (one block per batch,
-// FP64 block scan in chunks of the block size).
+// One batch's reservoir after a pass (one block per batch): the inclusive CDF
+// of its face weights (FP64 block scan in chunks of the block size), the status
+// of its chain, and the counters of the next pass zeroed (the reservoir that
+// the pass consumed becomes the next one's output; `next` the rays claimed).
+// live: chains still active after this pass, counted here so that the host can
+// stop queueing passes.  Three memsets and a status launch per pass went into
+// this kernel: the passes are short, and most of a solve was launches.
+struct SrmStepLaunch {
+    const double* faceW;   // [B][nF] of the reservoir filled by the pass
+    double* cdf;           // [B][nF]
+    uint32_t* usedCounts;  // [B][nF] the reservoir the pass consumed
+    double* usedW;
+    uint32_t* next;        // [B]
+    uint32_t* live;        // [4] active chains after pass p at p % 4; the next one is zeroed here
+    SrmChain* chain;       // [B]
+    uint32_t nF, pass, streak;
+    double tol;
+};
+
+__device__ void srmControl(SrmChain& ch, double cur, uint32_t pass, double tol, uint32_t streak);
+
 constexpr uint32_t kScanBlock = 1024u;
-__global__ void __launch_bounds__(kScanBlock) srmScanKernel(const double* faceW, double* cdf, uint32_t nF) {
+__global__ void __launch_bounds__(kScanBlock) srmStepKernel(const SrmStepLaunch S) {
     __shared__ double warpTot[kScanBlock / 32];
-    const double* in = faceW + size_t(blockIdx.x) * nF;
-    double* out = cdf + size_t(blockIdx.x) * nF;
+    const uint32_t nF = S.nF;
+    const double* in = S.faceW + size_t(blockIdx.x) * nF;
+    double* out = S.cdf + size_t(blockIdx.x) * nF;
+    uint32_t* usedCounts = S.usedCounts + size_t(blockIdx.x) * nF;
+    double* usedW = S.usedW + size_t(blockIdx.x) * nF;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double carry = 0.0;
     for (uint32_t base = 0; base < nF; base += kScanBlock) {
         const uint32_t k = base + threadIdx.x;
         double v = k < nF ? in[k] : 0.0;
+        if (k < nF) {
+            usedCounts[k] = 0u;
+            usedW[k] = 0.0;
+        }
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double n = __shfl_up_sync(0xffffffffu, v, o);
@@ -625,6 +651,13 @@ __global__ void __launch_bounds__(kScanBlock) srmScanKernel(const double* faceW,
         if (k < nF) out[k] = carry + v;
         carry += warpTot[kScanBlock / 32 - 1];
         __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        SrmChain& ch = S.chain[blockIdx.x];
+        srmControl(ch, out[nF - 1], S.pass, S.tol, S.streak);
+        S.next[blockIdx.x] = 0u;
+        if (ch.active) atomicAdd(S.live + (S.pass & 3u), 1u);
+        if (blockIdx.x == 0) S.live[(S.pass + 1u) & 3u] = 0u;
     }
 }
 
@@ -658,17 +691,12 @@ __global__ void srmSortKernel(const uint32_t* counts, double4* slot, uint32_t* l
     }
 }
 
-// Status of every batch's chain after a pass (include/core/forwardSrm.hpp:
+// Status of a batch's chain after a pass (include/core/forwardSrm.hpp:
 // 281-363): pass 0 opens the chain with the first reservoir's weight (none:
 // converged); later passes compare the new total weight with the previous
 // one: a growth streak of `streak` passes ends it as diverged, a relative
 // change below `tol` as stable, a weight below tol x the first as converged.
-__global__ void srmControlKernel(SrmChain* chain, const double* cdf, uint32_t nF, uint32_t B, uint32_t pass,
-                                 double tol, uint32_t streak) {
-    const uint32_t b = threadIdx.x;
-    if (b >= B) return;
-    const double cur = nF ? cdf[size_t(b) * nF + nF - 1] : 0.0;
-    SrmChain& ch = chain[b];
+__device__ void srmControl(SrmChain& ch, double cur, uint32_t pass, double tol, uint32_t streak) {
     if (pass == 0) {
         ch.grow = 0;
         ch.passes = 0;
@@ -901,6 +929,9 @@ struct hase_tet_context {
     DevBuf<double> resW[2], cdf;
     DevBuf<double4> resSlot[2];
     DevBuf<SrmChain> chain;
+    DevBuf<uint32_t> live;          // active chains of the last passes (srmStepKernel) ...
+    uint32_t* hLive = nullptr;      // ... and on the host (pinned)
+    cudaEvent_t srmEv[4] = {nullptr, nullptr, nullptr, nullptr};
 
     TetView view() const {
         TetView v{};
@@ -1146,6 +1177,9 @@ hase_status hase_tet_context_destroy(hase_tet_context* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (cudaEvent_t& e : c->ev)
         if (e) cudaEventDestroy(e);
+    for (cudaEvent_t& e : c->srmEv)
+        if (e) cudaEventDestroy(e);
+    if (c->hLive) cudaFreeHost(c->hLive);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return HASE_OK;
@@ -1292,6 +1326,10 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
         }
         HASE_CUDA(c->cdf.ensure(faces));
         HASE_CUDA(c->chain.ensure(B));
+        HASE_CUDA(c->live.ensure(4));
+        if (!c->hLive) HASE_CUDA(cudaMallocHost(&c->hLive, 4 * sizeof(uint32_t)));
+        for (cudaEvent_t& e : c->srmEv)
+            if (!e) HASE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (perSM < 1) return fail(HASE_CUDA_ERROR, "the ray kernel does not fit on an SM");
     const uint32_t resident = uint32_t(perSM) * c->numSMs;
@@ -1416,8 +1454,12 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
             } else {
                 // surface-reservoir chain: the source pass deposits into
                 // reservoir 0, reflected pass p reads reservoir (p - 1) % 2 and
-                // deposits into p % 2; every pass is queued, batches whose
-                // chain ended skip the rest on the device (no host sync)
+                // deposits into p % 2; batches whose chain ended skip the rest
+                // on the device.  The host stays one pass ahead of the count of
+                // active chains it waits for, so the device never idles and at
+                // most one pass runs after the last chain ended (8 live passes
+                // of 40 on a disc with total internal reflection: queueing all
+                // 40 took 2.9 ms of which the dead ones a fifth)
                 const size_t faces = size_t(B) * nF;
                 SrmLaunch& S = L.srm;
                 S.faces = c->bfaces.p;
@@ -1425,7 +1467,16 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
                 S.S = srmSlots;
                 S.cdf = c->cdf.p;
                 S.chain = c->chain.p;
+                HASE_CUDA(cudaMemsetAsync(c->resCounts[0].p, 0, faces * sizeof(uint32_t), c->stream));
+                HASE_CUDA(cudaMemsetAsync(c->resW[0].p, 0, faces * sizeof(double), c->stream));
+                HASE_CUDA(cudaMemsetAsync(c->live.p, 0, 4 * sizeof(uint32_t), c->stream));
                 for (uint32_t pass = 0; pass <= srmMaxIt; ++pass) {
+                    // the count of active chains two passes back: none left ends the queue
+                    // (the pass queued since then finds no active batch)
+                    if (pass >= 2) {
+                        HASE_CUDA(cudaEventSynchronize(c->srmEv[(pass - 2) & 3u]));
+                        if (c->hLive[(pass - 2) & 3u] == 0u) break;
+                    }
                     const int out = int(pass & 1u), in = 1 - out;
                     S.pass = pass;
                     S.outCounts = c->resCounts[out].p;
@@ -1436,10 +1487,7 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
                     S.inCounts = c->resCounts[in].p;
                     S.inSlot = c->resSlot[in].p;
                     S.inLam = c->resLam[in].p;
-                    HASE_CUDA(cudaMemsetAsync(S.outCounts, 0, faces * sizeof(uint32_t), c->stream));
-                    HASE_CUDA(cudaMemsetAsync(S.outFaceW, 0, faces * sizeof(double), c->stream));
                     if (pass > 0) {
-                        HASE_CUDA(cudaMemsetAsync(c->next.p, 0, B * sizeof(uint32_t), c->stream));
                         for (uint32_t b = 0; b < B; ++b) {
                             const Philox4 o = philox4x32_10(b, launch, pass, kTagFwdBatch, fw->rngSeed, kFwdKeyHi);
                             L.shift[b] = double(o.x) / 4294967296.0;
@@ -1453,11 +1501,14 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
                     HASE_CUDA(cudaGetLastError());
                     srmSortKernel<<<uint32_t((faces + 255) / 256), 256, 0, c->stream>>>(
                         S.outCounts, S.outSlot, S.outLam, S.outRay, srmSlots, faces);
-                    srmScanKernel<<<B, kScanBlock, 0, c->stream>>>(S.outFaceW, c->cdf.p, nF);
-                    srmControlKernel<<<1, kMaxBatches, 0, c->stream>>>(c->chain.p, c->cdf.p, nF, B, pass, srmTol,
-                                                                      srmStreak);
+                    const SrmStepLaunch step{S.outFaceW, c->cdf.p, c->resCounts[in].p, c->resW[in].p, c->next.p,
+                                             c->live.p, c->chain.p, nF, pass, srmStreak, srmTol};
+                    srmStepKernel<<<B, kScanBlock, 0, c->stream>>>(step);
                     HASE_CUDA(cudaGetLastError());
-                    res->kernelLaunches += 4;
+                    HASE_CUDA(cudaMemcpyAsync(c->hLive + (pass & 3u), c->live.p + (pass & 3u), sizeof(uint32_t),
+                                              cudaMemcpyDeviceToHost, c->stream));
+                    HASE_CUDA(cudaEventRecord(c->srmEv[pass & 3u], c->stream));
+                    res->kernelLaunches += 3;
                 }
                 chainRan = true;
             }
