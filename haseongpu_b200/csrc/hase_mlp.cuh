@@ -410,4 +410,8 @@ struct hase_proposal {
     hase::DevBuf<int> error;   // set by a kernel whose tensor-core wait timed out
     // training state
     hase::DevBuf<float> dparams, adamM, adamV, grad, loss;
+    // the rows of the last training batch, kept so that the calls of a
+    // fine-tuning loop do not allocate
+    hase::DevBuf<uint32_t> batchOffsets;
+    hase::DevBuf<float> batchFeatures, batchTargets, batchWeights, batchLogits, batchDl, lossHistory;
 };

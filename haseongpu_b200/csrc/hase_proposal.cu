@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -56,7 +57,6 @@ __device__ __forceinline__ float dsilu(float z) {
     return sg * (1.0f + z * (1.0f - sg));
 }
 
-// g[j] += sum over the tile's rows r of h[r][i0 + j] * dz[r][o] (j < 32) and
 // This thread's row of 64 values as bf16 row threadIdx.x of a canonical
 // K = 64 image at off (the A operand of the backward products).
 __device__ __forceinline__ void storeRowBf16(const Tile& T, uint32_t off, const float (&v)[kHid]) {
@@ -288,8 +288,12 @@ __global__ void __launch_bounds__(kTile, 2) mlpBackwardKernel(const TrainLaunch 
             float acc[kHid];
             loadCols<kHid>(T, TrainSmem::colGradW32, acc);
             const uint32_t lane = t & 31u, r = 16u * (t >> 5) + (lane & 15u);
-            float* g = P.grad + (lane < 16u ? kOffW3 : kOffW2) + r * kHid;
-            for (int n = 0; n < kHid; ++n) atomicAdd(g + n, acc[n]);
+            // four columns per reduction: the rows are 256-byte aligned, and
+            // every CTA adds its 8,192 sums to the same rows
+            float4* g = reinterpret_cast<float4*>(P.grad + (lane < 16u ? kOffW3 : kOffW2) + r * kHid);
+#pragma unroll
+            for (int n = 0; n < kHid / 4; ++n)
+                atomicAdd(g + n, make_float4(acc[4 * n], acc[4 * n + 1], acc[4 * n + 2], acc[4 * n + 3]));
         }
         flushGradient<kIn>(T, TrainSmem::colGradW1, P.grad + kOffW1, 1u, kHid, kFeat);
     }
@@ -326,13 +330,20 @@ __device__ __forceinline__ float blockReduce(float v, float* red, bool isMax) {
     __syncthreads();
     if (lane == 0) red[warp] = v;
     __syncthreads();
-    v = red[0];
-    for (int k = 1; k < int(blockDim.x >> 5); ++k) v = isMax ? fmaxf(v, red[k]) : v + red[k];
+    v = red[lane];  // 32 warps
+    for (int o = 16; o > 0; o >>= 1) {
+        const float w = __shfl_xor_sync(0xffffffffu, v, o);
+        v = isMax ? fmaxf(v, w) : v + w;
+    }
     return v;
 }
 
-__global__ void __launch_bounds__(256) groupStatsKernel(const StatsLaunch S) {
-    __shared__ float red[8];
+// One block of 1024 threads per group: a step has 8 to 16 groups of some
+// thousand rows, so the kernel is a chain of passes over one group's rows and
+// what counts is the rows per thread (44 us with 256 threads for 9,000 rows).
+constexpr uint32_t kStatsBlock = 1024;
+__global__ void __launch_bounds__(kStatsBlock) groupStatsKernel(const StatsLaunch S) {
+    __shared__ float red[kStatsBlock / 32];
     const uint32_t g = S.g0 + blockIdx.x;
     const uint32_t a = S.offsets[g] - S.rowBase, b = S.offsets[g + 1] - S.rowBase;
     float m = -INFINITY;
@@ -355,47 +366,47 @@ __global__ void __launch_bounds__(256) groupStatsKernel(const StatsLaunch S) {
     if (threadIdx.x == 0 && st > 0.0f) atomicAdd(S.loss, w * (lse - stl / st));
 }
 
-__global__ void adamKernel(float* p, float* m, float* v, const float* g, int n, float lr, float b1, float b2,
-                           float eps, float c1, float c2) {
+// One Adam step and the step's BF16 weight images and FP32 vector (the device
+// copy of packImages): thread i updates parameter i and writes it to its images,
+// and leaves the gradient zeroed for the next step.  The images' padding (input
+// features 12 .. 15) stays as uploadParams wrote it.
+__global__ void adamPackKernel(float* p, float* m, float* v, float* g, float lr, float b1, float b2, float eps,
+                               float c1, float c2, uint8_t* img, float* vec) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= HASE_PROPOSAL_PARAMS) return;
     const float gi = g[i];
+    g[i] = 0.0f;
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-// BF16 weight images and the f32 vector from the f32 master parameters
-// (the device copy of packImages).
-__global__ void packKernel(const float* p, uint8_t* img, float* vec) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    constexpr uint32_t n1 = kHid * kIn, n2 = kHid * kHid;
-    auto put = [&](uint32_t base, uint32_t n, uint32_t k, uint32_t K, float val) {
+    const float val = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = val;
+    const auto put = [&](uint32_t base, uint32_t n, uint32_t k, uint32_t K) {
         *reinterpret_cast<__nv_bfloat16*>(img + base + canonOffset(n, k, K)) = __float2bfloat16_rn(val);
     };
-    if (i < n1) {
-        const uint32_t n = i / kIn, k = i % kIn;
-        put(TrainSmem::w1, n, k, kIn, k < uint32_t(kFeat) ? p[kOffW1 + k * kHid + n] : 0.0f);
-    } else if (i < n1 + 4 * n2) {
-        const uint32_t j = i - n1, which = j / n2, n = (j % n2) / kHid, k = j % kHid;
-        if (which == 0) put(TrainSmem::w2, n, k, kHid, p[kOffW2 + k * kHid + n]);
-        else if (which == 1) put(TrainSmem::w3, n, k, kHid, p[kOffW3 + k * kHid + n]);
-        else if (which == 2) put(TrainSmem::w2b, n, k, kHid, p[kOffW2 + n * kHid + k]);
-        else put(TrainSmem::w3b, n, k, kHid, p[kOffW3 + n * kHid + k]);
-    } else if (i < n1 + 4 * n2 + uint32_t(kVecFloats)) {
-        const uint32_t j = i - n1 - 4 * n2;
-        float val;
-        if (j < uint32_t(kHid)) val = p[kOffB1 + j];
-        else if (j < 2u * kHid) val = p[kOffB2 + j - kHid];
-        else if (j < 3u * kHid) val = p[kOffB3 + j - 2 * kHid];
-        else if (j < 4u * kHid) val = __bfloat162float(__float2bfloat16_rn(p[kOffW4 + j - 3 * kHid]));
-        else val = p[kOffB4];
-        vec[j] = val;
+    if (i < kOffB1) {  // W1 [in][out]
+        put(TrainSmem::w1, uint32_t(i) % kHid, uint32_t(i) / kHid, kIn);
+    } else if (i < kOffW2) {
+        vec[i - kOffB1] = val;
+    } else if (i < kOffB2) {
+        const uint32_t r = uint32_t(i - kOffW2) / kHid, c = uint32_t(i - kOffW2) % kHid;
+        put(TrainSmem::w2, c, r, kHid);
+        put(TrainSmem::w2b, r, c, kHid);
+    } else if (i < kOffW3) {
+        vec[kHid + i - kOffB2] = val;
+    } else if (i < kOffB3) {
+        const uint32_t r = uint32_t(i - kOffW3) / kHid, c = uint32_t(i - kOffW3) % kHid;
+        put(TrainSmem::w3, c, r, kHid);
+        put(TrainSmem::w3b, r, c, kHid);
+    } else if (i < kOffW4) {
+        vec[2 * kHid + i - kOffB3] = val;
+    } else if (i < kOffB4) {
+        vec[3 * kHid + i - kOffW4] = __bfloat162float(__float2bfloat16_rn(val));
+    } else {
+        vec[4 * kHid] = val;
     }
 }
-constexpr uint32_t kPackThreads = kHid * kIn + 4 * kHid * kHid + kVecFloats;
 
 }  // namespace
 
@@ -574,9 +585,7 @@ namespace {
 struct DeviceBatch {
     uint32_t groups = 0, rows = 0;
     std::vector<uint32_t> offsets;
-    DevBuf<uint32_t> doffsets;
-    DevBuf<float> features, targets, weights, logits, dl;
-    bool hasWeights = false;
+    bool hasWeights = false;  // the rows are in the network's batch buffers
 };
 
 hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, DeviceBatch& d) {
@@ -588,24 +597,24 @@ hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, Device
     d.rows = b->offsets[b->groups];
     if (d.rows == 0) return fail(HASE_INVALID_ARGUMENT, "the batch has no rows");
     if (!b->features || !b->targets) return fail(HASE_INVALID_ARGUMENT, "features and targets are required");
-    for (uint32_t r = 0; r < d.rows; ++r)
-        if (!(b->targets[r] >= 0.0f) || !std::isfinite(b->targets[r]))
-            return fail(HASE_INVALID_ARGUMENT, "targets must be finite and >= 0");
+    bool valid = true;  // one flag over all rows: the loop has no exit and vectorises
+    for (uint32_t r = 0; r < d.rows; ++r) valid &= b->targets[r] >= 0.0f && b->targets[r] <= FLT_MAX;
+    if (!valid) return fail(HASE_INVALID_ARGUMENT, "targets must be finite and >= 0");
     d.offsets.assign(b->offsets, b->offsets + b->groups + 1);
     d.hasWeights = b->groupWeights != nullptr;
-    HASE_CUDA(d.doffsets.ensure(b->groups + 1));
-    HASE_CUDA(d.features.ensure(size_t(d.rows) * kFeat));
-    HASE_CUDA(d.targets.ensure(d.rows));
-    HASE_CUDA(d.logits.ensure(d.rows));
-    HASE_CUDA(d.dl.ensure(d.rows));
-    HASE_CUDA(cudaMemcpyAsync(d.doffsets.p, b->offsets, (b->groups + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
+    HASE_CUDA(net->batchOffsets.ensure(b->groups + 1));
+    HASE_CUDA(net->batchFeatures.ensure(size_t(d.rows) * kFeat));
+    HASE_CUDA(net->batchTargets.ensure(d.rows));
+    HASE_CUDA(net->batchLogits.ensure(d.rows));
+    HASE_CUDA(net->batchDl.ensure(d.rows));
+    HASE_CUDA(cudaMemcpyAsync(net->batchOffsets.p, b->offsets, (b->groups + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
                               net->stream));
-    HASE_CUDA(cudaMemcpyAsync(d.features.p, b->features, size_t(d.rows) * kFeat * sizeof(float),
+    HASE_CUDA(cudaMemcpyAsync(net->batchFeatures.p, b->features, size_t(d.rows) * kFeat * sizeof(float),
                               cudaMemcpyHostToDevice, net->stream));
-    HASE_CUDA(cudaMemcpyAsync(d.targets.p, b->targets, d.rows * sizeof(float), cudaMemcpyHostToDevice, net->stream));
+    HASE_CUDA(cudaMemcpyAsync(net->batchTargets.p, b->targets, d.rows * sizeof(float), cudaMemcpyHostToDevice, net->stream));
     if (d.hasWeights) {
-        HASE_CUDA(d.weights.ensure(b->groups));
-        HASE_CUDA(cudaMemcpyAsync(d.weights.p, b->groupWeights, b->groups * sizeof(float), cudaMemcpyHostToDevice,
+        HASE_CUDA(net->batchWeights.ensure(b->groups));
+        HASE_CUDA(cudaMemcpyAsync(net->batchWeights.p, b->groupWeights, b->groups * sizeof(float), cudaMemcpyHostToDevice,
                                   net->stream));
     }
     return HASE_OK;
@@ -619,14 +628,14 @@ hase_status lossGrad(hase_proposal* net, DeviceBatch& d, uint32_t g0, uint32_t g
     const uint32_t tiles = (rows + kTile - 1) / kTile;
     const uint32_t grid = std::min(tiles, 2u * net->numSMs);  // two CTAs per SM
     const uint32_t fgrid = std::min(tiles, net->numSMs * kMlpBlocksPerSM);
-    ForwardLaunch F{net->wimg.p, net->vec.p, d.features.p + size_t(r0) * kFeat, d.logits.p + r0, rows, net->error.p};
+    ForwardLaunch F{net->wimg.p, net->vec.p, net->batchFeatures.p + size_t(r0) * kFeat, net->batchLogits.p + r0, rows, net->error.p};
     mlpForwardKernel<<<fgrid, kTile, kSmemBytes, net->stream>>>(F);
     HASE_CUDA(cudaGetLastError());
-    StatsLaunch S{d.logits.p, d.targets.p, d.hasWeights ? d.weights.p : nullptr, d.doffsets.p, g0, 0u,
-                  1.0f / float(g1 - g0), d.dl.p, dLoss};
-    groupStatsKernel<<<g1 - g0, 256, 0, net->stream>>>(S);
+    StatsLaunch S{net->batchLogits.p, net->batchTargets.p, d.hasWeights ? net->batchWeights.p : nullptr, net->batchOffsets.p, g0, 0u,
+                  1.0f / float(g1 - g0), net->batchDl.p, dLoss};
+    groupStatsKernel<<<g1 - g0, kStatsBlock, 0, net->stream>>>(S);
     HASE_CUDA(cudaGetLastError());
-    TrainLaunch T{net->wimg.p, net->vec.p, d.features.p + size_t(r0) * kFeat, d.dl.p + r0, rows, dGrad,
+    TrainLaunch T{net->wimg.p, net->vec.p, net->batchFeatures.p + size_t(r0) * kFeat, net->batchDl.p + r0, rows, dGrad,
                   net->error.p};
     mlpBackwardKernel<<<grid, kTile, kTrainSmemBytes, net->stream>>>(T);
     HASE_CUDA(cudaGetLastError());
@@ -674,7 +683,7 @@ hase_status hase_proposal_train(hase_proposal* net, const hase_proposal_batch* b
     if (tr->groupsPerStep > d.groups) return fail(HASE_INVALID_ARGUMENT, "groupsPerStep exceeds the groups");
     const float b1 = tr->beta1 > 0.0f ? tr->beta1 : 0.9f, b2 = tr->beta2 > 0.0f ? tr->beta2 : 0.999f;
     const float eps = tr->epsilon > 0.0f ? tr->epsilon : 1e-8f;
-    DevBuf<float> hist;
+    DevBuf<float>& hist = net->lossHistory;
     HASE_CUDA(hist.ensure(tr->steps));
     HASE_CUDA(cudaMemsetAsync(hist.p, 0, tr->steps * sizeof(float), net->stream));
     HASE_CUDA(net->dparams.ensure(HASE_PROPOSAL_PARAMS));
@@ -684,19 +693,17 @@ hase_status hase_proposal_train(hase_proposal* net, const hase_proposal_batch* b
                               cudaMemcpyHostToDevice, net->stream));
     HASE_CUDA(cudaMemsetAsync(net->adamM.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
     HASE_CUDA(cudaMemsetAsync(net->adamV.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
+    HASE_CUDA(cudaMemsetAsync(net->grad.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
     const uint32_t blocks = d.groups / tr->groupsPerStep;
     double p1 = 1.0, p2 = 1.0;
     for (uint32_t step = 0; step < tr->steps; ++step) {
         const uint32_t g0 = (step % blocks) * tr->groupsPerStep, g1 = g0 + tr->groupsPerStep;
-        HASE_CUDA(cudaMemsetAsync(net->grad.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
         HASE_TRY(lossGrad(net, d, g0, g1, hist.p + step, net->grad.p));
         p1 *= b1;
         p2 *= b2;
-        adamKernel<<<(HASE_PROPOSAL_PARAMS + 255) / 256, 256, 0, net->stream>>>(
-            net->dparams.p, net->adamM.p, net->adamV.p, net->grad.p, HASE_PROPOSAL_PARAMS, tr->learningRate, b1, b2,
-            eps, float(1.0 - p1), float(1.0 - p2));
-        packKernel<<<(kPackThreads + 255) / 256, 256, 0, net->stream>>>(
-            net->dparams.p, reinterpret_cast<uint8_t*>(net->wimg.p), net->vec.p);
+        adamPackKernel<<<(HASE_PROPOSAL_PARAMS + 127) / 128, 128, 0, net->stream>>>(
+            net->dparams.p, net->adamM.p, net->adamV.p, net->grad.p, tr->learningRate, b1, b2, eps, float(1.0 - p1),
+            float(1.0 - p2), reinterpret_cast<uint8_t*>(net->wimg.p), net->vec.p);
         HASE_CUDA(cudaGetLastError());
     }
     HASE_CUDA(cudaMemcpyAsync(net->params.data(), net->dparams.p, HASE_PROPOSAL_PARAMS * sizeof(float),
