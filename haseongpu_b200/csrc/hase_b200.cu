@@ -284,30 +284,42 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
                 done = !(sOut > m.tolEnd);
                 sOut = done ? 0.0f : sOut;
                 if (COUNT) ++columns;
+                float n[LPL], fo[LPL];
+                int bits[LPL];
+                bool event = false;
 #pragma unroll
                 for (int g = 0; g < LPL; ++g) {
                     const float p = fmaf(sOut, inv[g], -0.5f);
                     const float r = p + kRound;
-                    const float n = r - kRound;  // levels left at the exit
-                    const float fo = p - n;
-                    while (n < nEvent[g]) {  // a bounce on the way
-                        const int s = bounce[g] & 1;
-                        if (bounce[g] & (4 << s)) lnR[g] += __logf(m.reflect ? __ldg(m.reflect + 2 * tk + s) : 0.0f);
-                        if (bounce[g] & 2) {
-                            bounce[g] = (bounce[g] & ~2) ^ 1;
-                            nEvent[g] -= float(layers);
-                        } else {
-                            if (bounce[g] & 16) {  // the second bounce of slice 4: from entry 0 to 2 layers - 1
-                                base[g] += 2 * layers;
-                                acc[g] += __ldg(&col[2 * layers].x) - __ldg(&col[0].x);
+                    n[g] = r - kRound;  // levels left at the exit
+                    fo[g] = p - n[g];
+                    bits[g] = __float_as_int(r);
+                    event = event || n[g] < nEvent[g];
+                }
+                if (event) {  // a bounce on the way of some line
+#pragma unroll
+                    for (int g = 0; g < LPL; ++g)
+                        while (n[g] < nEvent[g]) {
+                            const int s = bounce[g] & 1;
+                            if (bounce[g] & (4 << s)) lnR[g] += __logf(m.reflect ? __ldg(m.reflect + 2 * tk + s) : 0.0f);
+                            if (bounce[g] & 2) {
+                                bounce[g] = (bounce[g] & ~2) ^ 1;
+                                nEvent[g] -= float(layers);
+                            } else {
+                                if (bounce[g] & 16) {  // the second bounce of slice 4: from entry 0 to 2 layers - 1
+                                    base[g] += 2 * layers;
+                                    acc[g] += __ldg(&col[2 * layers].x) - __ldg(&col[0].x);
+                                }
+                                nEvent[g] = -1.0f;
                             }
-                            nEvent[g] = -1.0f;
                         }
-                    }
-                    entry[g] = __float_as_int(r) + base[g];
+                }
+#pragma unroll
+                for (int g = 0; g < LPL; ++g) {
+                    entry[g] = bits[g] + base[g];
                     const float2 out = __ldg(col + entry[g]);
-                    acc[g] += fmaf(in[g].y, f[g], fmaf(-out.y, fo, in[g].x - out.x));
-                    f[g] = fo;
+                    acc[g] += fmaf(in[g].y, f[g], fmaf(-out.y, fo[g], in[g].x - out.x));
+                    f[g] = fo[g];
                 }
                 if (!done) {
                     w = code;
