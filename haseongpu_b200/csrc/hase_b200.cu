@@ -1082,8 +1082,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
 // Launch shapes of rayKernel the autotuner chooses from: block size, idle
 // lanes that trigger a refill, the occupancy target (blocks per SM the
 // register budget is fitted to) and the triangle columns a lane walks per
-// step call (32 unless named).  Entry 0 is the default.  Single-medium shapes
-// also carry the kernels of the other walk modes.
+// step call (32 unless named).  Entry 0 is the default: 64 registers a thread
+// without spills beat five blocks of 48 with 50 to 110 bytes of them wherever
+// both were timed (5,470 mono samples 27.7 against 29.7 ms, 256 polychromatic
+// ones 4.66 / 4.86, 512 with grid weights 8.59 / 8.98, 5-sample query 21 us
+// both).  Single-medium shapes also carry the kernels of the other walk modes.
 struct RayVariant {
     void (*kernel)(RayLaunch);
     int block;
@@ -1095,6 +1098,7 @@ struct RayVariant {
     {rayKernel<B, R, M, false, false, C>, B, NAME, rayKernel<B, R, M, false, false, C, kWalkTable>, \
      rayKernel<B, R, M, false, false, C, kWalkBetaNoClad>}
 const RayVariant kRayVariants[] = {
+    HASE_RAY_SHAPE(512, 8, 2, 64, "block512_refill8_occ2_cols64"),
     HASE_RAY_SHAPE(256, 8, 5, kWalkColumns, "block256_refill8_occ5"),
     HASE_RAY_SHAPE(256, 4, 5, kWalkColumns, "block256_refill4_occ5"),
     HASE_RAY_SHAPE(256, 16, 5, kWalkColumns, "block256_refill16_occ5"),
@@ -1104,7 +1108,6 @@ const RayVariant kRayVariants[] = {
     HASE_RAY_SHAPE(128, 8, 12, kWalkColumns, "block128_refill8_occ12"),
     HASE_RAY_SHAPE(512, 8, 2, kWalkColumns, "block512_refill8_occ2"),
     HASE_RAY_SHAPE(256, 16, 5, 64, "block256_refill16_occ5_cols64"),
-    HASE_RAY_SHAPE(512, 8, 2, 64, "block512_refill8_occ2_cols64"),
 };
 #undef HASE_RAY_SHAPE
 constexpr uint32_t kNumRayVariants = sizeof(kRayVariants) / sizeof(kRayVariants[0]);
@@ -1114,6 +1117,7 @@ static_assert(kNumRayVariants <= 16, "variantBlocks holds 16 launch shapes");
 #define HASE_POOL_SHAPE(B, R, M, C, NAME) \
     {rayKernel<B, R, M, false, true, C>, B, NAME, nullptr, rayKernel<B, R, M, false, true, C, kWalkBetaNoClad>}
 const RayVariant kPoolVariants[] = {
+    HASE_POOL_SHAPE(512, 8, 2, 64, "block512_refill8_occ2_cols64"),
     HASE_POOL_SHAPE(256, 8, 5, kWalkColumns, "block256_refill8_occ5"),
     HASE_POOL_SHAPE(256, 4, 5, kWalkColumns, "block256_refill4_occ5"),
     HASE_POOL_SHAPE(256, 16, 5, kWalkColumns, "block256_refill16_occ5"),
@@ -1123,7 +1127,6 @@ const RayVariant kPoolVariants[] = {
     HASE_POOL_SHAPE(128, 8, 12, kWalkColumns, "block128_refill8_occ12"),
     HASE_POOL_SHAPE(512, 8, 2, kWalkColumns, "block512_refill8_occ2"),
     HASE_POOL_SHAPE(256, 16, 5, 64, "block256_refill16_occ5_cols64"),
-    HASE_POOL_SHAPE(512, 8, 2, 64, "block512_refill8_occ2_cols64"),
 };
 #undef HASE_POOL_SHAPE
 static_assert(sizeof(kPoolVariants) == sizeof(kRayVariants), "one batched variant per launch shape");
@@ -2993,7 +2996,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             const RayVariant& shape = local ? (logOut ? localLog : kLocalVariant) : (logOut ? logVariant : kRayVariants[variant]);
             const uint64_t totalItems = uint64_t(nActive) * items;
             void (*const kern)(RayLaunch) = walk == kWalkTable ? shape.mono : (walk == kWalkBetaNoClad ? shape.noClad : shape.kernel);
-            uint32_t resident = c->variantBlocks[walk][variant];
+            uint32_t resident = logOut ? c->persistentBlocks : c->variantBlocks[walk][variant];
             if (local) {  // occupancy of the local kernel itself
                 int perSM = 0, sms = 0;
                 HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, shape.block, 0));

@@ -173,6 +173,13 @@ enum WalkMode {
     kWalkBetaNoClad = 2,   // as kWalkBeta for a medium without cladding prisms (beta is never NaN)
 };
 
+// Reciprocal with the hardware approximation (1 ulp; subnormal inputs give inf).
+__device__ __forceinline__ float rcpApprox(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Initialise a ray from the start point, given as its offset (dx, dy, dz)
 // from the image point (Sx, Sy, kImg*h), in physical layer `layer`.
 // Returns |start - image|^2.
@@ -181,8 +188,11 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     const float h = m.h;
     if (dz == 0.0f) dz = 1e-6f * h;  // a ray inside a level plane: nudge it off the plane
     const float D2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float D = sqrtf(D2);
-    const float inv = 1.0f / D;
+    // 1 / D to its last bit or two: the approximation and one Newton step (a
+    // rounded square root and a rounded division took three times the instructions)
+    const float i0 = rsqrtf(D2);
+    const float inv = fmaf(0.5f * i0, fmaf(-D2 * i0, i0, 1.0f), i0);
+    const float D = D2 * inv;
     r.row = layer * int(m.T);
     r.reflLeft = expectedReflections(slice);
     r.s = D;
@@ -194,7 +204,7 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     r.uy = dy * inv;
     r.uz = dz * inv;
     // moving toward the image: down (layer step -1) when uz > 0, up (+1) otherwise
-    const float hu = __fdividef(h, r.uz);
+    const float hu = h * rcpApprox(r.uz);
     r.hOverUz = r.uz > 0.0f ? -hu : hu;
     const int zl0 = r.uz > 0.0f ? kImg - layer : layer + 1 - kImg;
     r.zl = float(zl0);
@@ -250,13 +260,6 @@ __device__ __forceinline__ double rayMeanGain(const Ray& r, const float2* spec, 
         sum += __expf(fminf(fmaf(ab.x - r.A, r.Jb, (r.B - ab.y) * Lg), 80.0f));
     }
     return e * double(sum) / double(nL);
-}
-
-// Reciprocal with the hardware approximation (1 ulp; subnormal inputs give inf).
-__device__ __forceinline__ float rcpApprox(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 // Exit parameter s = e / d of one window edge for a ray along -u to the sample:
@@ -340,7 +343,7 @@ __device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ra
                 return kDropped;
             }
         }
-        gb = __ldg(gcol + r.row + t);
+        if (plane) gb = __ldg(gcol + r.row + t);
         sz = r.zl * r.hOverUz;
         plane = plane && sz > cut;
         next = plane ? sz : sEnd;
