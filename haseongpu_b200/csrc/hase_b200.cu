@@ -115,7 +115,7 @@ void invariantDivisor(uint32_t d, uint32_t& mul, uint32_t& shift) {
 struct ImportanceLaunch {
     MeshView m;
     uint32_t firstSample, rows, slices, nW;
-    const float2* line;  // [T][phases layers]: lineTableKernel
+    const float2* line;  // [T][phases layers]: meshTablesKernel
     float* lnw;   // [rows][nW]
     const uint32_t* rowList;  // rows to compute (blockIdx.y indexes it), or null: rows 0 .. rows - 1
     const uint8_t* rowFlag;   // batched media: only rows with rowFlag[flagBase + row] set are computed (or null)
@@ -128,8 +128,8 @@ struct ImportanceLaunch {
     uint32_t divLm, divLs;  // floor(x / layers) = (x * divLm) >> divLs
 };
 
-// The lines' table: per triangle the gain along z in the unfolded direction a
-// line moves in.  Entry i of triangle t belongs to the i-th layer of the
+// The lines' table (TableJob::line): per triangle the gain along z in the unfolded
+// direction a line moves in.  Entry i of triangle t belongs to the i-th layer of the
 // sequence down, up, down (phases x layers entries, i falling along a line's
 // way: phase 0 is a line moving down in layer i, phase 1 one moving up in
 // layer 2 layers - 1 - i, phase 2 down again) and holds (F, g): g of the layer's
@@ -139,24 +139,41 @@ struct ImportanceLaunch {
 // any stretch of a triangle is then a difference of two F + g (position -
 // middle), whatever the number of levels and reflections in between.
 // Without reflections a line stays in phase 0 or 1 (phases = 2).
-__global__ void lineTableKernel(const float* gainBeta, float A, float B, float cladAbs, uint32_t T, uint32_t layers,
-                                uint32_t phases, float2* line) {
+struct TableJob {
+    const float* gainBeta;  // [layers][T], NaN in cladding
+    float A, B, cladAbs;
+    uint32_t T, layers, phases;
+    float2* line;           // [T][phases layers] or null
+    float* walk;            // [T][layers]: the ray walk's table (MeshView::walkTab)
+    int walkGain;           // its values: g, or beta
+};
+
+// A medium's tables for one solve, one thread per triangle; jobs: one medium per
+// blockIdx.y (a batch), or null: `one`.
+__global__ void meshTablesKernel(const TableJob* jobs, TableJob one) {
+    const TableJob J = jobs ? jobs[blockIdx.y] : one;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
+    if (t >= J.T) return;
+    const float absorb = fminf(J.cladAbs, 1e30f);  // finite: F is a difference
     double total = 0.0;
-    for (uint32_t l = 0; l < layers; ++l) {
-        const float b = gainBeta[size_t(l) * T + t];
-        total += double((b == b) ? fmaf(b, A, -B) : -fminf(cladAbs, 1e30f));  // finite: F is a difference
+    float* walk = J.walk + size_t(t) * J.layers;
+    for (uint32_t l = 0; l < J.layers; ++l) {
+        const float b = __ldg(J.gainBeta + size_t(l) * J.T + t);
+        const float g = (b == b) ? fmaf(b, J.A, -J.B) : -J.cladAbs;
+        walk[l] = J.walkGain ? g : b;
+        total += double((b == b) ? g : -absorb);
     }
-    float2* out = line + size_t(t) * phases * layers;
-    double F = -0.5 * double(phases) * total;
-    for (uint32_t i = 0; i < phases * layers; ++i) {
-        const uint32_t r = i % layers, l = (i / layers) & 1u ? layers - 1u - r : r;
-        const float b = gainBeta[size_t(l) * T + t];
-        const float g = (b == b) ? fmaf(b, A, -B) : -fminf(cladAbs, 1e30f);
-        out[i] = make_float2(float(F + 0.5 * double(g)), g);
-        F += double(g);
-    }
+    if (!J.line) return;
+    float2* out = J.line + size_t(t) * J.phases * J.layers;
+    double F = -0.5 * double(J.phases) * total;
+    for (uint32_t ph = 0, i = 0; ph < J.phases; ++ph)
+        for (uint32_t r = 0; r < J.layers; ++r, ++i) {
+            const uint32_t l = ph & 1u ? J.layers - 1u - r : r;
+            const float b = __ldg(J.gainBeta + size_t(l) * J.T + t);
+            const float g = (b == b) ? fmaf(b, J.A, -J.B) : -absorb;
+            out[i] = make_float2(float(F + 0.5 * double(g)), g);
+            F += double(g);
+        }
 }
 
 __host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slices == 1 ? 2u : 3u; }
@@ -2169,7 +2186,7 @@ struct hase_context {
     float tirCos2[2] = {-1.0f, -1.0f};
     DevBuf<float4> tri, win, geo;
     DevBuf<int4> verts;
-    DevBuf<float2> line;  // the importance lines' table of the last solve (lineTableKernel)
+    DevBuf<float2> line;  // the importance lines' table of the last solve (meshTablesKernel)
     // local proposal (hase_context_set_local_proposal): per point the K
     // triangles nearest to it (by centroid distance, nearest first) and the
     // same set by ascending index; the far proposal's prefix of beta V over
@@ -2188,7 +2205,8 @@ struct hase_context {
     uint64_t farVersion = 0;
     DevBuf<float2> centroid, points, spec;
     DevBuf<float> gainBeta, srcBeta, reflect;
-    DevBuf<float> gTab;  // g of every prism for the spectrally averaged (A, B) of the last solve
+    DevBuf<float> gTab;  // g of every prism for the spectrally averaged (A, B) of the last solve (far prior)
+    DevBuf<float> walkTab;  // MeshView::walkTab of the last solve
     // workspace
     DevBuf<float> lnw;
     DevBuf<uint32_t> q, offsets, activeA, activeB, pDrop;
@@ -2227,7 +2245,7 @@ struct hase_context {
         v.geo = geo.p;
         v.verts = verts.p;
         v.centroid = centroid.p;
-        v.gainBeta = gainBeta.p;
+        v.walkTab = walkTab.p;
         v.gTab = gTab.p;
         v.srcBeta = srcBeta.p;
         v.points = points.p;
@@ -2392,13 +2410,17 @@ void localFields(hase_context* c, ImportanceLaunch& il) {
     il.K = c->localK;
 }
 
-// The importance lines' table of the context's beta for the averaged (A, B),
-// built on stream s.
-hase_status buildLineTable(hase_context* c, double A, double B, uint32_t slices, cudaStream_t s) {
-    const uint32_t phases = linePhases(slices);
-    HASE_CUDA(c->line.ensure(size_t(c->P) * phases));
-    lineTableKernel<<<(c->T + 127) / 128, 128, 0, s>>>(c->gainBeta.p, float(A), float(B), float(c->cladAbs), c->T,
-                                                       c->layers, phases, c->line.p);
+// The tables of the context's beta for the averaged (A, B): the ray walk's (g
+// for walkGain, else beta) and, for slices > 0, the importance lines'.
+TableJob tableJob(const hase_context* c, double A, double B, uint32_t slices, bool walkGain, float2* line, float* walk) {
+    return TableJob{c->gainBeta.p, float(A), float(B), float(c->cladAbs), c->T, c->layers, linePhases(slices),
+                    slices ? line : nullptr, walk, walkGain ? 1 : 0};
+}
+
+hase_status buildTables(hase_context* c, double A, double B, uint32_t slices, bool walkGain) {
+    if (slices) HASE_CUDA(c->line.ensure(size_t(c->P) * linePhases(slices)));
+    meshTablesKernel<<<(c->T + 127) / 128, 128, 0, c->stream>>>(
+        nullptr, tableJob(c, A, B, slices, walkGain, c->line.p, c->walkTab.p));
     HASE_CUDA(cudaGetLastError());
     return HASE_OK;
 }
@@ -2683,7 +2705,8 @@ hase_status hase_context_create(const hase_mesh_desc* d, const hase_spectrum_des
     if ((st = up(c->verts, ht.verts)) != HASE_OK) return cleanup(st);
     if ((st = up(c->centroid, ht.centroid)) != HASE_OK) return cleanup(st);
     if ((st = up(c->points, ht.points)) != HASE_OK) return cleanup(st);
-    if (c->gainBeta.ensure(c->P) != cudaSuccess || c->srcBeta.ensure(c->P) != cudaSuccess)
+    if (c->gainBeta.ensure(c->P) != cudaSuccess || c->srcBeta.ensure(c->P) != cudaSuccess ||
+        c->walkTab.ensure(c->P) != cudaSuccess)
         return cleanup(fail(HASE_OUT_OF_MEMORY, "beta tables"));
     if (d->reflectivities) {
         std::vector<float> r(2 * size_t(c->T));
@@ -2862,19 +2885,16 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     std::vector<double> hRse;
     std::vector<uint32_t> hTot;
 
-    // the ray walk of a monochromatic solve and the far prior read each
-    // prism's g from a table, the importance walks their lines' integrals
-    // (rebuilt here: beta may have changed since the last solve)
+    // the walks' tables (rebuilt here: beta may have changed since the last solve)
     // walk mode of the ray launches (the logging launches keep the general walk)
     const int walk = logOut ? kWalkBeta : (nLambda == 1 ? kWalkTable : (c->hasClad ? kWalkBeta : kWalkBetaNoClad));
-    HASE_CUDA(c->gTab.ensure(c->P));
-    gainTableKernel<<<(c->P + 255) / 256, 256, 0, c->stream>>>(c->gainBeta.p, float(meanA), float(meanB),
-                                                               float(c->cladAbs), c->P, c->gTab.p);
-    HASE_CUDA(cudaGetLastError());
     const bool walks = la ? la->fallbackVariance > 0.0f : !gridWeights;
-    if (walks) HASE_TRY(buildLineTable(c, meanA, meanB, slices, c->stream));
+    HASE_TRY(buildTables(c, meanA, meanB, walks ? slices : 0u, walk == kWalkTable));
     ProposalView fpv{};
-    if (farPrior) {  // the far prior's cell gains for this solve's g, and the layer-averaged coarse gain grid
+    if (farPrior) {  // the far prior's g of every prism, its cell gains, and the layer-averaged coarse gain grid
+        HASE_CUDA(c->gTab.ensure(c->P));
+        gainTableKernel<<<(c->P + 255) / 256, 256, 0, c->stream>>>(c->gainBeta.p, float(meanA), float(meanB),
+                                                                   float(c->cladAbs), c->P, c->gTab.p);
         const uint32_t n = c->farCells * c->layers;
         farGainKernel<<<(n + 255) / 256, 256, 0, c->stream>>>(c->cellStart.p, c->cellTris.p, c->farCells, c->gTab.p, c->T,
                                                               c->layers, c->gCell.p);
@@ -2895,7 +2915,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
     res->totalMilliseconds = 0;
     res->passes = 0;
     res->unconvergedSamples = 0;
-    res->kernelLaunches = (farPrior ? 3 : 1) + (walks ? 1 : 0);  // the tables (and the far prior's cell gains and gain grid)
+    res->kernelLaunches = farPrior ? 4 : 1;  // the tables (and the far prior's g, cell gains and gain grid)
     uint64_t droppedTotal = 0;
 
     for (uint32_t b0 = 0; b0 < nS; b0 += rows) {
@@ -3598,7 +3618,7 @@ hase_status hase_importance_weights(hase_context* c, uint32_t firstSample, uint3
     HASE_CUDA(q.ensure(size_t(count) * nW));
     HASE_CUDA(off.ensure(size_t(count) * (nW + 1)));
     HASE_CUDA(Q.ensure(count));
-    HASE_TRY(buildLineTable(c, meanA, meanB, slices, c->stream));
+    HASE_TRY(buildTables(c, meanA, meanB, slices, false));
     ImportanceLaunch il{c->view(), firstSample, count, slices, nW, c->line.p, lnw.p};
     localFields(c, il);
     HASE_CUDA(launchImportance(il, c->layers, c->T, c->Np, count, c->stream));
@@ -3658,7 +3678,7 @@ hase_status hase_importance_crossings(hase_context* c, uint32_t firstSample, uin
     HASE_CUDA(lnw.ensure(size_t(count) * nW));
     HASE_CUDA(n.ensure(1));
     HASE_CUDA(cudaMemsetAsync(n.p, 0, sizeof(unsigned long long), c->stream));
-    HASE_TRY(buildLineTable(c, 0.0, 0.0, slices, c->stream));
+    HASE_TRY(buildTables(c, 0.0, 0.0, slices, false));
     ImportanceLaunch il{c->view(), firstSample, count, slices, nW, c->line.p, lnw.p};
     localFields(c, il);
     il.crossings = n.p;
@@ -3807,6 +3827,7 @@ hase_status hase_trace_rays(hase_context* c, uint32_t n, const float* start, con
     HASE_CUDA(cudaMemcpyAsync(dSli.p, slice, n * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
     const float A = float(c->nTot * (c->sigmaE[wavelength] + c->sigmaA[wavelength]));
     const float B = float(c->nTot * c->sigmaA[wavelength]);
+    HASE_TRY(buildTables(c, 0.0, 0.0, 0u, false));
     TraceLaunch tl{c->view(), n, dStart.p, dTri.p, dLev.p, dSam.p, dSli.p, A, B, dLn.p, dDist.p, dDrop.p};
     traceKernel<<<(n + 127) / 128, 128, 0, c->stream>>>(tl);
     HASE_CUDA(cudaGetLastError());
@@ -3964,6 +3985,7 @@ hase_status hase_estimate_sample_noalloc(hase_context* c, uint32_t sample, const
 
     // The scratch keeps the previous call's contents: clear what must start at zero.
     HASE_CUDA(cudaMemsetAsync(small, 0, 256, c->stream));  // Q, active = {row 0}, counters, accumulators
+    HASE_TRY(buildTables(c, 0.0, 0.0, 0u, false));  // beta in the walk table: a launch, no allocation
     const MeshView mv = c->view();
     MapLaunch ml{deviceWeights, 0, 1, active, uint32_t(nW), rays, nullptr, sample, 0u, rngSeed, 0u,
                  nullptr, q, Q, offsets};
@@ -4003,6 +4025,9 @@ struct hase_batch {
     std::vector<cudaEvent_t> ev;  // timing events recorded inside the graphs
     DevBuf<float> lnw, prior;
     DevBuf<unsigned char> rowState;  // RowView
+    DevBuf<float2> line;          // the media's tables (meshTablesKernel)
+    DevBuf<float> walkTab;
+    DevBuf<TableJob> tableJobs;
     DevBuf<uint8_t> rowFlag;      // rows restarting with the importance weights (learned solve)
     DevBuf<uint32_t> q, offsets, activeA, activeB, pDrop;
     DevBuf<unsigned int> counts;  // [0], [1]: active rows (alternating), [2]: item counter, [3 ..]: per pass
@@ -4195,12 +4220,32 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     // media views and spectra
     HASE_CUDA(b->spec.ensure(specPool.size()));
     HASE_CUDA(b->inst.ensure(count));
+    // every medium's tables in the batch's own buffers
+    const auto walksOf = [&](uint32_t i) { return net ? fallbackVariance > 0.0f : !media[i].c->gridProposal; };
+    std::vector<size_t> lineAt(count), walkAt(count);
+    size_t lineEntries = 0, walkEntries = 0;
+    uint32_t maxT = 0;
+    for (uint32_t i = 0; i < count; ++i) {
+        const hase_context* c = media[i].c;
+        lineAt[i] = lineEntries;
+        walkAt[i] = walkEntries;
+        lineEntries += walksOf(i) ? size_t(c->P) * linePhases(slices) : 0;
+        walkEntries += c->P;
+        maxT = std::max(maxT, c->T);
+    }
+    HASE_CUDA(b->line.ensure(lineEntries));
+    HASE_CUDA(b->walkTab.ensure(walkEntries));
+    HASE_CUDA(b->tableJobs.ensure(count));
+    std::vector<TableJob> jobs(count);
     std::vector<InstanceView> views(count);
     for (uint32_t i = 0; i < count; ++i) {
         const hase_context* c = media[i].c;
+        jobs[i] = tableJob(c, media[i].meanA, media[i].meanB, walksOf(i) ? slices : 0u, false, b->line.p + lineAt[i],
+                           b->walkTab.p + walkAt[i]);
         InstanceView& v = views[i];
         std::memset(&v, 0, sizeof(v));
         v.m = c->view();
+        v.m.walkTab = b->walkTab.p + walkAt[i];
         v.spec = b->spec.p + specBase[i];
         v.nLambda = media[i].nLambda;
         v.nW = media[i].nW;
@@ -4211,7 +4256,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                               b->stream));
     HASE_CUDA(cudaMemcpyAsync(b->inst.p, views.data(), count * sizeof(InstanceView), cudaMemcpyHostToDevice,
                               b->stream));
-    uint32_t tableLaunches = 0;
+    HASE_CUDA(cudaMemcpyAsync(b->tableJobs.p, jobs.data(), count * sizeof(TableJob), cudaMemcpyHostToDevice,
+                              b->stream));
     // learned proposal: one feature view per medium (coarse gain grid on the medium's context)
     std::vector<ProposalView> pviews;
     uint32_t proposalGrid = 0;
@@ -4237,14 +4283,11 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     // the views' gain grids are built on each context's own stream: finished
     // before the batch's stream reads them
     for (uint32_t i = 0; i < count; ++i) HASE_CUDA(cudaStreamSynchronize(media[i].c->stream));
-
-    // the importance lines' tables (on the batch's stream: every medium of a
-    // context has the same spectrum, so a context listed twice gets the same table)
-    for (uint32_t i = 0; i < count; ++i)
-        if (net ? fallbackVariance > 0.0f : !media[i].c->gridProposal) {
-            HASE_TRY(buildLineTable(media[i].c, media[i].meanA, media[i].meanB, slices, b->stream));
-            ++tableLaunches;
-        }
+    for (uint32_t i = 0; i < count; i += 65535) {
+        const uint32_t n = std::min(count - i, 65535u);
+        meshTablesKernel<<<dim3((maxT + 127) / 128, n), 128, 0, b->stream>>>(b->tableJobs.p + i, TableJob{});
+        HASE_CUDA(cudaGetLastError());
+    }
 
     // rows of every medium, cut into workspace chunks
     struct Chunk {
@@ -4307,7 +4350,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     }
 
     hase_batch_stats st{};
-    st.kernelLaunches = tableLaunches;
+    st.kernelLaunches = 1;  // the media's tables
     st.rows = uint32_t(all.size());
     st.chunks = uint32_t(chunks.size());
     std::vector<uint32_t> unconvergedOf(count, 0), passesOf(count, 0);
@@ -4338,7 +4381,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
                 const BatchMedium& md = media[i];
                 const hase_context* c = md.c;
                 const uint32_t segRows = uint32_t(e - r);
-                ImportanceLaunch il{views[i].m, all[r].sample, segRows, slices, md.nW, c->line.p,
+                ImportanceLaunch il{views[i].m, all[r].sample, segRows, slices, md.nW, b->line.p + lineAt[i],
                                     b->lnw.p + all[r].w, nullptr, flag, uint32_t(r - ch.r0)};
                 HASE_CUDA(launchImportance(il, c->layers, c->T, c->Np, segRows, b->stream));
                 ++kernels;

@@ -73,7 +73,11 @@ struct MeshView {
     const float4* geo;       // [T][2]
     const int4* verts;       // [T] point ids of the triangle's vertices (w unused)
     const float2* centroid;  // [T]
-    const float* gainBeta;   // [P] beta, NaN in cladding prisms (walk)
+    // [T][layers] the ray walk's value of each prism (WalkMode): g, or beta with
+    // NaN in cladding prisms.  Triangle-major: the rays of a warp cross the same
+    // triangles at different heights, so their reads share a column's one or two
+    // lines; layer-major they were up to one line per lane.
+    const float* walkTab;
     const float* gTab;       // [P] g of each prism for the solve's averaged (A, B) (a monochromatic solve: its pair)
     const float* srcBeta;    // [P] beta (source weight)
     const float2* points;    // [Np]
@@ -131,14 +135,14 @@ __device__ __forceinline__ float reflectFactor(const MeshView& m, uint32_t t, in
 }
 
 // One ray in flight.  The walk runs in the unfolded z coordinate (reflection
-// images); `row` is the prism-index offset (physical layer x T) of the current
-// unfolded layer and `rstep` the offset of the next physical layer toward the
-// image point, +T or -T (it flips at every reflection), so no division, modulo
-// or multiplication is needed per crossing.
+// images); `row` is the physical layer of the current unfolded layer and
+// `rstep` the step to the next physical layer toward the image point, +1 or -1
+// (it flips at every reflection), so no division or modulo is needed per
+// crossing.
 struct Ray {
     uint32_t w;     // edge window: 4 triangle + first slot (MeshView::win)
-    int row;        // physical layer of the current unfolded layer, times T
-    int rstep;      // +T / -T
+    int row;        // physical layer of the current unfolded layer
+    int rstep;      // +1 / -1
     int reflLeft;   // reflections the slice still implies
     int steps;      // triangles left minus the first zl: with the current zl, the crossings so far (raySteps)
     float s;        // remaining distance to the image point
@@ -168,8 +172,8 @@ enum StepResult { kContinue = 0, kDone = 1, kDropped = 2 };
 // (rayMeanGain); for the reference pair it is G itself, bit for bit as the
 // table walk gives it.
 enum WalkMode {
-    kWalkBeta = 0,         // beta from m.gainBeta; cladding prisms (NaN beta) add to Lc
-    kWalkTable = 1,        // g from m.gTab (a monochromatic solve: the table is built for its pair)
+    kWalkBeta = 0,         // m.walkTab holds beta; cladding prisms (NaN beta) add to Lc
+    kWalkTable = 1,        // m.walkTab holds g (a monochromatic solve: the table is built for its pair)
     kWalkBetaNoClad = 2,   // as kWalkBeta for a medium without cladding prisms (beta is never NaN)
 };
 
@@ -193,7 +197,7 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     const float i0 = rsqrtf(D2);
     const float inv = fmaf(0.5f * i0, fmaf(-D2 * i0, i0, 1.0f), i0);
     const float D = D2 * inv;
-    r.row = layer * int(m.T);
+    r.row = layer;
     r.reflLeft = expectedReflections(slice);
     r.s = D;
     r.G = 0.0f;
@@ -209,7 +213,7 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     const int zl0 = r.uz > 0.0f ? kImg - layer : layer + 1 - kImg;
     r.zl = float(zl0);
     r.steps = -zl0;
-    r.rstep = r.uz > 0.0f ? -int(m.T) : int(m.T);
+    r.rstep = r.uz > 0.0f ? -1 : 1;
     r.A = A;
     r.B = B;
     // the first window leaves out an edge the ray does not move out through
@@ -305,17 +309,17 @@ __device__ __forceinline__ bool reflectRay(const MeshView& m, Ray& r, uint32_t t
 //   loop over the planes ran for the whole warp as often as its worst lane
 //   needed.
 // Crossings are counted by the columns and zl, the step bound is checked once
-// per call, and kWalkTable walks the table of g = beta A - B (m.gTab).
+// per call, and kWalkTable walks a table of g = beta A - B.
 // Boundary edges are never exits: the 2-D mesh is convex and the target lies
 // in it, so only rounding could route a ray across one.
 template <int K = 1, int WALK = kWalkBeta>
 __device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ray& r) {
-    const float* gcol = WALK == kWalkTable ? m.gTab : m.gainBeta;
     const float4* win = m.win;
+    const auto value = [&](uint32_t t) { return __ldg(m.walkTab + (t * m.layers + uint32_t(r.row))); };
     float4 a = __ldg(win + r.w), b = __ldg(win + r.w + 1);
     // beta (kWalkTable: g) of the current prism, issued with the record so
     // that its latency overlaps the edge tests
-    float gb = __ldg(gcol + r.row + (r.w >> 2));
+    float gb = value(r.w >> 2);
 #pragma unroll 1
     for (int k = 0; k < K; ++k) {
         const uint32_t t = r.w >> 2;
@@ -337,13 +341,13 @@ __device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ra
             r.row += r.rstep;
             r.zl += 1.0f;
         }
-        if (uint32_t(r.row) >= m.P) {
+        if (uint32_t(r.row) >= m.layers) {
             if (!reflectRay(m, r, t)) {
                 r.steps += k;
                 return kDropped;
             }
         }
-        if (plane) gb = __ldg(gcol + r.row + t);
+        if (plane) gb = value(t);
         sz = r.zl * r.hOverUz;
         plane = plane && sz > cut;
         next = plane ? sz : sEnd;
@@ -352,11 +356,11 @@ __device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ra
         while (plane) {
             r.row += r.rstep;
             r.zl += 1.0f;
-            if (uint32_t(r.row) >= m.P && !reflectRay(m, r, t)) {
+            if (uint32_t(r.row) >= m.layers && !reflectRay(m, r, t)) {
                 r.steps += k;
                 return kDropped;
             }
-            gb = __ldg(gcol + r.row + t);
+            gb = value(t);
             sz = r.zl * r.hOverUz;
             plane = sz > cut;
             next = plane ? sz : sEnd;
@@ -368,7 +372,7 @@ __device__ __forceinline__ int stepRay(const MeshView& m, float Sx, float Sy, Ra
             return kDone;
         }
         r.w = code;
-        gb = __ldg(gcol + r.row + (code >> 2));
+        gb = value(code >> 2);
     }
     r.steps += K;
     // the step bound, once per call: a call walks at most K columns of at most
