@@ -2040,7 +2040,10 @@ __global__ void farGainKernel(const uint32_t* cellStart, const uint32_t* cellTri
 
 // Per sample row of a chunk: the inclusive FP64 prefix over (cell, slice)
 // pairs of the far prior's weights w_cj = sum_l term_clj (FP32, layers in
-// order, empty layers skipped: the terms localSource's layer scan adds).  One block per row, 256 pairs per step, warp-shuffle scans.
+// order, empty layers skipped: the terms localSource's layer scan adds).  One
+// block per row, one thread per cell: its position, g_mid and the layers' mass
+// and gain serve all SL slices, 256 cells per step, warp-shuffle scans.
+template <int SL>
 __global__ void __launch_bounds__(256) farRowKernel(FarRowLaunch L) {
     __shared__ double wsum[8];
     const uint32_t row = blockIdx.x, sample = L.firstSample + row;
@@ -2048,28 +2051,37 @@ __global__ void __launch_bounds__(256) farRowKernel(FarRowLaunch L) {
     const int ls = int(sample / L.Np);
     const float gs = farSampleGain(L.gTab, L.cand, L.K, L.T, L.layers, sample % L.Np, ls);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t nE = L.C * L.slices;
-    double* out = L.rowCdf + size_t(row) * nE;
+    int kImg[SL];
+#pragma unroll
+    for (int j = 0; j < SL; ++j) kImg[j] = imageLevel(ls, int(L.layers), uint32_t(j));
+    double* out = L.rowCdf + size_t(row) * L.C * SL;
     double carry = 0.0;
-    for (uint32_t e0 = 0; e0 < nE; e0 += 256) {
-        const uint32_t e = e0 + threadIdx.x;
-        float w = 0.0f;
-        if (e < nE) {
-            const uint32_t c = e / L.slices, j = e - c * L.slices;
-            const int kImg = imageLevel(ls, int(L.layers), j);
+    for (uint32_t c0 = 0; c0 < L.C; c0 += 256) {
+        const uint32_t c = c0 + threadIdx.x;
+        float w[SL];
+#pragma unroll
+        for (int j = 0; j < SL; ++j) w[j] = 0.0f;
+        if (c < L.C) {
             const float4 cl = L.cell[c];
             const float* mass = L.cellMass + size_t(c) * L.layers;
             const float* gc = L.gCell + size_t(c) * L.layers;
             const float gmid = farMidGain(L, S, cl.x, cl.y);
-            if (j == 0) L.gMid[size_t(row) * L.C + c] = gmid;
+            L.gMid[size_t(row) * L.C + c] = gmid;
             for (uint32_t l = 0; l < L.layers; ++l) {
-                const float mcl = mass[l];
+                const float mcl = __ldg(mass + l);
                 if (!(mcl > 0.0f)) continue;
-                const float d2 = farDistance2(cl, S, int(l), kImg, L.h);
-                w += farTerm(farSliceFactor(L.refl, j, int(l) - kImg, L.h, d2), mcl, d2, farMeanGain(gc[l], gs, gmid));
+                const float g = farMeanGain(__ldg(gc + l), gs, gmid);
+#pragma unroll
+                for (int j = 0; j < SL; ++j) {
+                    const float d2 = farDistance2(cl, S, int(l), kImg[j], L.h);
+                    w[j] += farTerm(farSliceFactor(L.refl, uint32_t(j), int(l) - kImg[j], L.h, d2), mcl, d2, g);
+                }
             }
         }
-        double x = double(w);
+        double x = 0.0;
+#pragma unroll
+        for (int j = 0; j < SL; ++j) x += double(w[j]);
+        const double own = x;
         for (int o = 1; o < 32; o <<= 1) {
             const double y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
@@ -2081,7 +2093,14 @@ __global__ void __launch_bounds__(256) farRowKernel(FarRowLaunch L) {
             if (k < warp) base += wsum[k];
             block += wsum[k];
         }
-        if (e < nE) out[e] = base + x;
+        if (c < L.C) {
+            double at = base + (x - own);
+#pragma unroll
+            for (int j = 0; j < SL; ++j) {
+                at += double(w[j]);
+                out[size_t(c) * SL + j] = at;
+            }
+        }
         carry += block;
         __syncthreads();
     }
@@ -2959,7 +2978,8 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             fl.y0 = fpv.y0;
             fl.invCell = fpv.invCell;
             farSlicePrior(c, fl.refl);
-            farRowKernel<<<nRows, 256, 0, c->stream>>>(fl);
+            if (slices == 1) farRowKernel<1><<<nRows, 256, 0, c->stream>>>(fl);
+            else farRowKernel<5><<<nRows, 256, 0, c->stream>>>(fl);
             res->kernelLaunches += 1;
         }
         HASE_CUDA(cudaGetLastError());
