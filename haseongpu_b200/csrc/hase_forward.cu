@@ -18,8 +18,9 @@
 //                  division per crossing).  Tally: weight G (e^{gl} - 1)/g split
 //                  to the cell's four material vertices by the segment-midpoint
 //                  barycentric weights, straight into device memory or (on
-//                  request) into a per-block shared-memory vertex histogram of
-//                  the block's batch, flushed once per block.
+//                  request, or with reflections where it fits) into a
+//                  per-block shared-memory vertex histogram of the block's
+//                  batch, flushed once per block.
 //   fwdFinalizeKernel  one thread per cell: vertex -> cell density through
 //                  the lumped material-vertex volumes, estimate
 //                  S B_tot / (N V) N_tot / tau, batch-mean relative error,
@@ -1318,18 +1319,24 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
     const uint32_t C = c->C, Np = c->Np;
     const size_t nV = 2 * size_t(Np);
     const size_t histBytes = nV * sizeof(double);
-    // Automatic: device memory. A block-wide histogram leaves one block of 8 warps
-    // per SM and costs its clearing and flush; the tallies carried along a ray
-    // leave one reduction per crossing, which L2 takes from 24 warps per SM with
-    // less trouble. Measured at every size where a histogram fits: 18 x 10 disc
-    // (164 KB), 2,000 rays 0.227 ms shared against 0.201 ms, 100,000 0.49 / 0.28,
-    // 4M 12.7 / 5.9; 8 x 6 disc (21 KB), 5,000 rays 0.120 / 0.103, 4M 5.6 / 5.3.
-    const bool smem = fw->tallyMode == 2;
+    // Automatic, without reflections: device memory. A block-wide histogram leaves
+    // one block of 8 warps per SM and costs its clearing and flush; the tallies
+    // carried along a ray leave one reduction per crossing, which L2 takes from 24
+    // warps per SM with less trouble. Measured at every size where a histogram
+    // fits: 18 x 10 disc (164 KB), 2,000 rays 0.227 ms shared against 0.201 ms,
+    // 100,000 0.49 / 0.28, 4M 12.7 / 5.9; 8 x 6 disc (21 KB), 5,000 rays 0.120 /
+    // 0.103, 4M 5.6 / 5.3. With reflections the histogram where it fits, although
+    // device memory is faster there too (18 x 10, 5,000 rays 2.28 / 1.54 ms): which
+    // deposits an overflowing reservoir keeps depends on the order in which they
+    // arrive, and 24 warps per SM bring them in another order than 8 (2 of 67 small
+    // chains then moved phi by up to 1e-4; none does with the histogram, and none
+    // with slots enough for every deposit).
+    const bool srm = fw->useReflections != 0;
+    const bool smem = fw->tallyMode == 2 || (fw->tallyMode == 0 && srm && histBytes <= kMaxHistogramBytes);
     if (smem && histBytes > kMaxHistogramBytes)
         return fail(HASE_INVALID_ARGUMENT, "shared-memory tallies need 2 * numberOfPoints * 8 <= %zu bytes",
                     kMaxHistogramBytes);
     int perSM = 0;
-    const bool srm = fw->useReflections != 0;
     if (smem) {
         HASE_CUDA(cudaFuncSetAttribute(fwdRayKernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(histBytes)));
