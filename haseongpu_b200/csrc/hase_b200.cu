@@ -39,7 +39,7 @@
 #include <mutex>
 #include <new>
 #include <string>
-#include <unordered_map>
+#include <utility>
 #include <vector>
 
 using namespace hase;
@@ -1896,8 +1896,13 @@ hase_status buildHostTables(const hase_mesh_desc* d, HostTables& h, double& exte
         extent = std::max(extent, std::max(std::fabs(d->points[2 * i]), std::fabs(d->points[2 * i + 1])));
     }
     std::vector<int32_t> nbr(3 * size_t(T), -1);
-    std::unordered_map<uint64_t, uint32_t> open;  // edge key -> 3*t + e
-    open.reserve(3 * size_t(T));
+    // edge key -> 3 t + e of the triangle that still waits for its neighbour there
+    // (kNone: none), by linear probing (a node-based map: creation 5 to 10% longer,
+    // 4.92 against 4.45 ms for 9,600 triangles x 29 layers)
+    constexpr uint32_t kNone = 0xffffffffu;
+    uint32_t bits = 4;
+    while ((uint64_t(1) << bits) < 6 * uint64_t(T)) ++bits;
+    std::vector<std::pair<uint64_t, uint32_t>> open(size_t(1) << bits, {~uint64_t(0), kNone});
     for (uint32_t t = 0; t < T; ++t) {
         const uint32_t* v = d->triangles + 3 * size_t(t);
         for (int e = 0; e < 3; ++e)
@@ -1917,15 +1922,18 @@ hase_status buildHostTables(const hase_mesh_desc* d, HostTables& h, double& exte
             ny[e] = -orient * ex * inv;
             c[e] = nx[e] * d->points[2 * a] + ny[e] * d->points[2 * a + 1];
             const uint64_t key = (uint64_t(std::min(a, b)) << 32) | std::max(a, b);
-            auto it = open.find(key);
-            if (it == open.end()) {
-                open.emplace(key, 3 * t + e);
+            size_t at = size_t((key * 0x9E3779B97F4A7C15ull) >> (64 - bits));
+            while (open[at].first != key && open[at].first != ~uint64_t(0)) at = (at + 1) & (open.size() - 1);
+            uint32_t& waiting = open[at].second;
+            open[at].first = key;
+            if (waiting == kNone) {
+                waiting = 3 * t + e;
             } else {
-                const uint32_t other = it->second;
+                const uint32_t other = waiting;
                 if (nbr[other] != -1) return fail(HASE_INVALID_ARGUMENT, "edge shared by more than two triangles");
                 nbr[3 * t + e] = int32_t(other);
                 nbr[other] = int32_t(3 * t + e);
-                open.erase(it);
+                waiting = kNone;
             }
         }
         h.tri[3 * t + 0] = make_float4(float(nx[0]), float(ny[0]), float(c[0]), float(nx[1]));
