@@ -46,7 +46,7 @@ sys.path.insert(0, str(REPO))
 METRIC = ("phi-ASE time to per-sample relative error <= threshold on 1 B200, as sample points solved per second "
           "(rays/s alongside)")
 FP32_INSTR_PER_CROSSING = 24   # stated per-crossing FP32 instruction count
-BYTES_PER_CROSSING = 52        # triangle record 48 B + prism beta 4 B
+BYTES_PER_CROSSING = 36        # a triangle's window of two edges 32 B + prism value 4 B
 SMS = 148
 LANES_PER_SM = 128
 MLP_FLOP_PER_PAIR = 2 * (12 * 64 + 64 * 64 + 64 * 64 + 64 * 1)  # 18,048 FLOP per (sample, prism) inference
@@ -419,8 +419,7 @@ def measure_importance(args, local, rank=0, world=1, nested=False):
                          "traffic": None, "fp32_issue_peak": r_fp32, "l2_gather_peak": r_l2,
                          "l2_read_gbs_live": l2, "clock_mhz": f_clk / 1e6, "peak_source": peak_kind},
             "importance_roofline": {"bound": "fp32_issue" if r_fp32 <= r_l2 else "l2_gather",
-                                    "kernel": "importanceTeamKernel" if tuned.importanceLayers == 0
-                                    else f"importanceKernel<{tuned.importanceLayers}>",
+                                    "kernel": "importanceTeamKernel",
                                     "achieved": imp_crossings / (imp_ms * 1e-3), "peak": roof, "unit": "crossings/s",
                                     "frac": imp_crossings / (imp_ms * 1e-3) / roof,
                                     "fp32_issue_frac": imp_crossings / (imp_ms * 1e-3) / r_fp32,
