@@ -410,6 +410,7 @@ struct hase_proposal {
     hase::DevBuf<int> error;   // set by a kernel whose tensor-core wait timed out
     // training state
     hase::DevBuf<float> dparams, adamM, adamV, grad, loss;
+    hase::DevBuf<float> gradRows, groupLoss;  // a step's sums: one gradient row per CTA, one loss term per group
     // the rows of the last training batch, kept so that the calls of a
     // fine-tuning loop do not allocate
     hase::DevBuf<uint32_t> batchOffsets;

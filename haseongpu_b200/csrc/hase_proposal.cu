@@ -143,7 +143,7 @@ __device__ __forceinline__ void tileRowSum(const Tile& T, float x, float& acc) {
     __syncthreads();
 }
 
-// Adds this thread's row of an M = 64 weight-gradient accumulator (TMEM
+// Writes this thread's row of an M = 64 weight-gradient accumulator (TMEM
 // column `col`, `cols` columns; lanes 0-15 of each warp hold rows 16 warp +
 // lane) to grad[base + row * rowStride + n * colStride] for n < keep.
 template <int COLS>
@@ -153,8 +153,11 @@ __device__ __forceinline__ void flushGradient(const Tile& T, uint32_t col, float
     loadCols<COLS>(T, col, acc);
     const uint32_t lane = threadIdx.x & 31u, row = 16u * (threadIdx.x >> 5) + lane;
     if (lane < 16u)
-        for (int n = 0; n < keep; ++n) atomicAdd(grad + row * rowStride + uint32_t(n) * colStride, acc[n]);
+        for (int n = 0; n < keep; ++n) grad[row * rowStride + uint32_t(n) * colStride] = acc[n];
 }
+
+// Floats between the gradient rows of two CTAs (a multiple of 4: 16-byte stores).
+constexpr uint32_t kGradStride = (HASE_PROPOSAL_PARAMS + 3u) / 4u * 4u;
 
 struct TrainLaunch {
     const uint4* wimg;      // forward + backward images
@@ -162,7 +165,7 @@ struct TrainLaunch {
     const float* features;  // [rows][kFeat]
     const float* dl;        // [rows]: dLoss / dlogit
     uint32_t rows;
-    float* grad;            // [HASE_PROPOSAL_PARAMS], accumulated
+    float* grad;            // [gridDim.x][kGradStride]: every CTA's sums
     int* error;
 };
 
@@ -172,8 +175,11 @@ struct TrainLaunch {
 // weight-gradient product (h2^T dz3, h1^T dz2, dz1^T x: the activation and dz
 // images read as MN-major operands) that accumulates in TMEM over all tiles
 // of the CTA; the bias sums run on the CUDA cores meanwhile.  Two CTAs per SM
-// (256 TMEM columns each, TrainSmem).  The CTA adds its gradients to `grad`
-// once.
+// (256 TMEM columns each, TrainSmem).  The CTA writes its sums to its own row
+// of `grad` once; gradientSum adds the rows in a fixed order.  (Adding them to
+// one row by atomics made the order of 296 sums a matter of which CTA came
+// first, and the parameters after 20 Adam steps by 7e-4 of their norm, up to
+// 1e-2 in one of 160 runs.)
 __global__ void __launch_bounds__(kTile, 2) mlpBackwardKernel(const TrainLaunch P) {
     extern __shared__ uint8_t dynSmem[];
     Tile T;
@@ -281,35 +287,32 @@ __global__ void __launch_bounds__(kTile, 2) mlpBackwardKernel(const TrainLaunch 
         fenceBeforeSync();
         if (!__syncthreads_and(T.ok)) break;
     }
-    if (accumulate) {
+    // gridDim.x <= tiles: every CTA had a tile, so its accumulators hold one
+    float* grad = P.grad + size_t(blockIdx.x) * kGradStride;
+    {
         // g_W3 (lanes 0-15) and g_W2 (lanes 16-31) as [in][out] rows (row =
         // input) from the interleaved block; g_W1^T as [out][in] rows
-        {
-            float acc[kHid];
-            loadCols<kHid>(T, TrainSmem::colGradW32, acc);
-            const uint32_t lane = t & 31u, r = 16u * (t >> 5) + (lane & 15u);
-            // four columns per reduction: the rows are 256-byte aligned, and
-            // every CTA adds its 8,192 sums to the same rows
-            float4* g = reinterpret_cast<float4*>(P.grad + (lane < 16u ? kOffW3 : kOffW2) + r * kHid);
+        float acc[kHid];
+        loadCols<kHid>(T, TrainSmem::colGradW32, acc);
+        const uint32_t lane = t & 31u, r = 16u * (t >> 5) + (lane & 15u);
+        float4* g = reinterpret_cast<float4*>(grad + (lane < 16u ? kOffW3 : kOffW2) + r * kHid);
 #pragma unroll
-            for (int n = 0; n < kHid / 4; ++n)
-                atomicAdd(g + n, make_float4(acc[4 * n], acc[4 * n + 1], acc[4 * n + 2], acc[4 * n + 3]));
-        }
-        flushGradient<kIn>(T, TrainSmem::colGradW1, P.grad + kOffW1, 1u, kHid, kFeat);
+        for (int n = 0; n < kHid / 4; ++n) g[n] = make_float4(acc[4 * n], acc[4 * n + 1], acc[4 * n + 2], acc[4 * n + 3]);
     }
+    flushGradient<kIn>(T, TrainSmem::colGradW1, grad + kOffW1, 1u, kHid, kFeat);
     if (ih == 0) {
-        atomicAdd(P.grad + kOffB1 + o, gb1);
-        atomicAdd(P.grad + kOffB2 + o, gb2);
-        atomicAdd(P.grad + kOffB3 + o, gb3);
-        atomicAdd(P.grad + kOffW4 + o, gw4);
+        grad[kOffB1 + o] = gb1;
+        grad[kOffB2 + o] = gb2;
+        grad[kOffB3 + o] = gb3;
+        grad[kOffW4 + o] = gw4;
     }
-    if (t == 0) atomicAdd(P.grad + kOffB4, gb4);
+    if (t == 0) grad[kOffB4] = gb4;
     tileEnd<TrainSmem>(T, P.error);
 }
 
 // Softmax statistics of group g (rows off[g] .. off[g+1] of the step, minus
 // rowBase): lse, and dl_r = w_g / G (exp(l_r - lse) - t_r / sum t); the group's
-// cross entropy w_g (lse - sum t l / sum t) / G is added to *loss.
+// cross entropy w_g (lse - sum t l / sum t) / G goes to groupLoss[g - g0].
 struct StatsLaunch {
     const float* logits;
     const float* targets;
@@ -318,7 +321,7 @@ struct StatsLaunch {
     uint32_t g0, rowBase;
     float invGroups;
     float* dl;
-    float* loss;
+    float* groupLoss;
 };
 
 __device__ __forceinline__ float blockReduce(float v, float* red, bool isMax) {
@@ -390,19 +393,64 @@ __global__ void __launch_bounds__(kStatsBlock) groupStatsKernel(const StatsLaunc
             if (r + k * kStatsBlock < b)
                 S.dl[r + k * kStatsBlock] = st > 0.0f ? w * (__expf(l[k] - m - lse) - t[k] / st) : 0.0f;
     }
-    if (threadIdx.x == 0 && st > 0.0f) atomicAdd(S.loss, w * (lse - stl / st));
+    if (threadIdx.x == 0) S.groupLoss[blockIdx.x] = st > 0.0f ? w * (lse - stl / st) : 0.0f;
 }
 
-// One Adam step and the step's BF16 weight images and FP32 vector (the device
-// copy of packImages): thread i updates parameter i and writes it to its images,
-// and leaves the gradient zeroed for the next step.  The images' padding (input
-// features 12 .. 15) stays as uploadParams wrote it.
-__global__ void adamPackKernel(float* p, float* m, float* v, float* g, float lr, float b1, float b2, float eps,
-                               float c1, float c2, uint8_t* img, float* vec) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= HASE_PROPOSAL_PARAMS) return;
-    const float gi = g[i];
-    g[i] = 0.0f;
+// The sums of a step: a parameter's gradient from the CTAs' rows and the loss
+// from the groups' terms, both in FP64 and in a fixed order, so that a call
+// repeats itself bit for bit.  A block sums 32 parameters with kSumLanes threads
+// each (thread y takes rows y, y + kSumLanes, ..., loads of a warp 128 bytes of
+// one row); the kernel reads 296 x 37 KB from L2.  A step of 73,008 rows takes
+// 94.2 us, 98.4 with the atomics.
+struct StepSums {
+    const float* rows;       // [nRows][kGradStride]
+    const float* groupLoss;  // [nGroups]
+    float* loss;             // the step's loss
+    uint32_t nRows, nGroups;
+};
+constexpr uint32_t kSumParams = 32, kSumLanes = 16;
+constexpr uint32_t kSumBlocks = (HASE_PROPOSAL_PARAMS + kSumParams - 1) / kSumParams;
+
+// The gradient of parameter blockIdx.x kSumParams + threadIdx.x, for the threads
+// with threadIdx.y = 0.  All threads; block 0 also writes the loss.
+__device__ __forceinline__ float gradientSum(const StepSums& S) {
+    __shared__ double part[kSumLanes][kSumParams];
+    const uint32_t i = blockIdx.x * kSumParams + threadIdx.x;
+    double sum = 0.0;
+    if (i < HASE_PROPOSAL_PARAMS) {
+#pragma unroll 8
+        for (uint32_t r = threadIdx.y; r < S.nRows; r += kSumLanes) sum += double(__ldg(S.rows + size_t(r) * kGradStride + i));
+    }
+    part[threadIdx.y][threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.y == 0)
+#pragma unroll
+        for (uint32_t y = 1; y < kSumLanes; ++y) sum += part[y][threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.y == 1) {
+        double l = 0.0;
+        for (uint32_t g = threadIdx.x; g < S.nGroups; g += 32) l += double(S.groupLoss[g]);
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (threadIdx.x == 0) *S.loss = float(l);
+    }
+    return float(sum);
+}
+
+__global__ void __launch_bounds__(kSumParams * kSumLanes) gradientSumKernel(const StepSums S, float* g) {
+    const float gi = gradientSum(S);
+    const uint32_t i = blockIdx.x * kSumParams + threadIdx.x;
+    if (threadIdx.y == 0 && i < HASE_PROPOSAL_PARAMS) g[i] = gi;
+}
+
+// One Adam step on the step's sums, and its BF16 weight images and FP32 vector
+// (the device copy of packImages): a parameter's thread updates it and writes
+// it to its images.  The images' padding (input features 12 .. 15) stays as
+// uploadParams wrote it.
+__global__ void __launch_bounds__(kSumParams * kSumLanes)
+    adamPackKernel(const StepSums S, float* p, float* m, float* v, float lr, float b1, float b2, float eps, float c1,
+                   float c2, uint8_t* img, float* vec) {
+    const float gi = gradientSum(S);
+    const int i = blockIdx.x * kSumParams + threadIdx.x;
+    if (threadIdx.y != 0 || i >= HASE_PROPOSAL_PARAMS) return;
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
@@ -647,22 +695,26 @@ hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, Device
     return HASE_OK;
 }
 
-// Loss (added to *dLoss) and gradient (added to dGrad) of groups [g0, g1).
-hase_status lossGrad(hase_proposal* net, DeviceBatch& d, uint32_t g0, uint32_t g1, float* dLoss, float* dGrad) {
+// The CTAs' gradient rows and the groups' loss terms of groups [g0, g1); out:
+// what sums them (no rows: a gradient and a loss of zero).
+hase_status lossGrad(hase_proposal* net, DeviceBatch& d, uint32_t g0, uint32_t g1, float* dLoss, StepSums& out) {
     const uint32_t r0 = d.offsets[g0], r1 = d.offsets[g1];
     const uint32_t rows = r1 - r0;
+    out = StepSums{net->gradRows.p, net->groupLoss.p, dLoss, 0u, 0u};
     if (rows == 0) return HASE_OK;
     const uint32_t tiles = (rows + kTile - 1) / kTile;
     const uint32_t grid = std::min(tiles, 2u * net->numSMs);  // two CTAs per SM
     const uint32_t fgrid = std::min(tiles, net->numSMs * kMlpBlocksPerSM);
+    out.nRows = grid;
+    out.nGroups = g1 - g0;
     ForwardLaunch F{net->wimg.p, net->vec.p, net->batchFeatures.p + size_t(r0) * kFeat, net->batchLogits.p + r0, rows, net->error.p};
     mlpForwardKernel<<<fgrid, kTile, kSmemBytes, net->stream>>>(F);
     HASE_CUDA(cudaGetLastError());
     StatsLaunch S{net->batchLogits.p, net->batchTargets.p, d.hasWeights ? net->batchWeights.p : nullptr, net->batchOffsets.p, g0, 0u,
-                  1.0f / float(g1 - g0), net->batchDl.p, dLoss};
+                  1.0f / float(g1 - g0), net->batchDl.p, net->groupLoss.p};
     groupStatsKernel<<<g1 - g0, kStatsBlock, 0, net->stream>>>(S);
     HASE_CUDA(cudaGetLastError());
-    TrainLaunch T{net->wimg.p, net->vec.p, net->batchFeatures.p + size_t(r0) * kFeat, net->batchDl.p + r0, rows, dGrad,
+    TrainLaunch T{net->wimg.p, net->vec.p, net->batchFeatures.p + size_t(r0) * kFeat, net->batchDl.p + r0, rows, net->gradRows.p,
                   net->error.p};
     mlpBackwardKernel<<<grid, kTile, kTrainSmemBytes, net->stream>>>(T);
     HASE_CUDA(cudaGetLastError());
@@ -674,8 +726,7 @@ hase_status prepareTraining(hase_proposal* net) {
     HASE_CUDA(cudaFuncSetAttribute(mlpForwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)));
     HASE_CUDA(
         cudaFuncSetAttribute(mlpBackwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTrainSmemBytes)));
-    HASE_CUDA(net->grad.ensure(HASE_PROPOSAL_PARAMS));
-    HASE_CUDA(net->loss.ensure(1));
+    HASE_CUDA(net->gradRows.ensure(size_t(2u * net->numSMs) * kGradStride));
     return HASE_OK;
 }
 
@@ -688,9 +739,13 @@ hase_status hase_proposal_loss_grad(hase_proposal* net, const hase_proposal_batc
     HASE_TRY(prepareTraining(net));
     DeviceBatch d;
     HASE_TRY(uploadBatch(net, batch, d));
-    HASE_CUDA(cudaMemsetAsync(net->grad.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
-    HASE_CUDA(cudaMemsetAsync(net->loss.p, 0, sizeof(float), net->stream));
-    HASE_TRY(lossGrad(net, d, 0, d.groups, net->loss.p, net->grad.p));
+    HASE_CUDA(net->grad.ensure(HASE_PROPOSAL_PARAMS));
+    HASE_CUDA(net->loss.ensure(1));
+    HASE_CUDA(net->groupLoss.ensure(d.groups));
+    StepSums sums;
+    HASE_TRY(lossGrad(net, d, 0, d.groups, net->loss.p, sums));
+    gradientSumKernel<<<kSumBlocks, dim3(kSumParams, kSumLanes), 0, net->stream>>>(sums, net->grad.p);
+    HASE_CUDA(cudaGetLastError());
     HASE_CUDA(cudaMemcpyAsync(grad, net->grad.p, HASE_PROPOSAL_PARAMS * sizeof(float), cudaMemcpyDeviceToHost,
                               net->stream));
     HASE_CUDA(cudaMemcpyAsync(loss, net->loss.p, sizeof(float), cudaMemcpyDeviceToHost, net->stream));
@@ -712,7 +767,7 @@ hase_status hase_proposal_train(hase_proposal* net, const hase_proposal_batch* b
     const float eps = tr->epsilon > 0.0f ? tr->epsilon : 1e-8f;
     DevBuf<float>& hist = net->lossHistory;
     HASE_CUDA(hist.ensure(tr->steps));
-    HASE_CUDA(cudaMemsetAsync(hist.p, 0, tr->steps * sizeof(float), net->stream));
+    HASE_CUDA(net->groupLoss.ensure(tr->groupsPerStep));
     HASE_CUDA(net->dparams.ensure(HASE_PROPOSAL_PARAMS));
     HASE_CUDA(net->adamM.ensure(HASE_PROPOSAL_PARAMS));
     HASE_CUDA(net->adamV.ensure(HASE_PROPOSAL_PARAMS));
@@ -720,16 +775,16 @@ hase_status hase_proposal_train(hase_proposal* net, const hase_proposal_batch* b
                               cudaMemcpyHostToDevice, net->stream));
     HASE_CUDA(cudaMemsetAsync(net->adamM.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
     HASE_CUDA(cudaMemsetAsync(net->adamV.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
-    HASE_CUDA(cudaMemsetAsync(net->grad.p, 0, HASE_PROPOSAL_PARAMS * sizeof(float), net->stream));
     const uint32_t blocks = d.groups / tr->groupsPerStep;
     double p1 = 1.0, p2 = 1.0;
     for (uint32_t step = 0; step < tr->steps; ++step) {
         const uint32_t g0 = (step % blocks) * tr->groupsPerStep, g1 = g0 + tr->groupsPerStep;
-        HASE_TRY(lossGrad(net, d, g0, g1, hist.p + step, net->grad.p));
+        StepSums sums;
+        HASE_TRY(lossGrad(net, d, g0, g1, hist.p + step, sums));
         p1 *= b1;
         p2 *= b2;
-        adamPackKernel<<<(HASE_PROPOSAL_PARAMS + 127) / 128, 128, 0, net->stream>>>(
-            net->dparams.p, net->adamM.p, net->adamV.p, net->grad.p, tr->learningRate, b1, b2, eps, float(1.0 - p1),
+        adamPackKernel<<<kSumBlocks, dim3(kSumParams, kSumLanes), 0, net->stream>>>(
+            sums, net->dparams.p, net->adamM.p, net->adamV.p, tr->learningRate, b1, b2, eps, float(1.0 - p1),
             float(1.0 - p2), reinterpret_cast<uint8_t*>(net->wimg.p), net->vec.p);
         HASE_CUDA(cudaGetLastError());
     }

@@ -101,3 +101,26 @@ def test_training_learns_a_known_proposal():
     assert np.all(np.isfinite(hist))
     assert loss0 - entropy > 0.3
     assert loss1 - entropy < 0.1 * (loss0 - entropy), (loss0, loss1, entropy)
+
+
+@pytest.mark.parametrize("sizes", [[1], [100, 28], [200, 0, 129], [2000] * 8, [19_000, 18_889], [9_126] * 8])
+def test_identical_training_calls_return_identical_bits(sizes):
+    """The gradient's and the loss's sums have one order: one tile of 128 rows, fewer tiles than CTAs, one more row than
+    the 296 CTAs' first tiles and several tiles each, and an empty group."""
+    rng = np.random.default_rng(len(sizes))
+    off = _groups(rng, sizes)
+    f = rng.normal(size=(off[-1], 12)).astype(np.float32)
+    t = (rng.random(off[-1]) ** 2).astype(np.float32)
+    per = 8 if len(sizes) == 8 else 1
+    runs, grads = [], []
+    for _ in range(3):
+        with _net(seed=4) as net:
+            grads.append(net.loss_grad(off, f, t))
+            loss = net.train(off, f, t, steps=20, groups_per_step=per, learning_rate=1e-3)
+            runs.append((np.asarray(loss), net.params))
+    for loss, params in runs[1:]:
+        np.testing.assert_array_equal(loss, runs[0][0])
+        np.testing.assert_array_equal(params, runs[0][1])
+    for l, g in grads[1:]:
+        assert l == grads[0][0]
+        np.testing.assert_array_equal(g, grads[0][1])
