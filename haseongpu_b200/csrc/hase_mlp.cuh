@@ -411,8 +411,6 @@ struct hase_proposal {
     // training state
     hase::DevBuf<float> dparams, adamM, adamV, grad, loss;
     hase::DevBuf<float> gradRows, groupLoss;  // a step's sums: one gradient row per CTA, one loss term per group
-    // the rows of the last training batch, kept so that the calls of a
-    // fine-tuning loop do not allocate
-    hase::DevBuf<uint32_t> batchOffsets;
-    hase::DevBuf<float> batchFeatures, batchTargets, batchWeights, batchLogits, batchDl, lossHistory;
+    hase::DevBuf<float> lossHistory;
+    hase::DevBuf<unsigned char> batchRows;  // the last call's rows (DeviceBatch)
 };

@@ -124,3 +124,22 @@ def test_identical_training_calls_return_identical_bits(sizes):
     for l, g in grads[1:]:
         assert l == grads[0][0]
         np.testing.assert_array_equal(g, grads[0][1])
+
+
+def test_rows_of_a_large_batch_are_given_back():
+    """1.3 million rows (78 MB) do not stay with the network; the rows of a small call may (at most 64 MB)."""
+    import torch
+
+    rng = np.random.default_rng(2)
+    off = _groups(rng, [650_000, 650_000])
+    f = rng.normal(size=(off[-1], 12)).astype(np.float32)
+    t = rng.random(off[-1]).astype(np.float32)
+    with _net() as net:
+        small = net.loss_grad(_groups(rng, [500, 500]), f[:1000], t[:1000])
+        before = torch.cuda.mem_get_info()[0]
+        net.loss_grad(off, f, t)
+        after = torch.cuda.mem_get_info()[0]
+        again = net.loss_grad(_groups(rng, [500, 500]), f[:1000], t[:1000])
+    assert before - after < 8 << 20
+    assert small[0] == again[0]
+    np.testing.assert_array_equal(small[1], again[1])
