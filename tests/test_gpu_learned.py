@@ -216,3 +216,23 @@ def test_fallback_restarts_samples_with_the_importance_weights(small, trained):
     assert np.mean(np.abs(z) < 4.0) > 0.95
     none = ctx.calc_phi_ase_learned(net, fallbackVariance=1e9, **kw)
     assert none.fallbackSamples == 0 and np.all(none.totalRays == 80000)
+
+
+def test_features_come_in_bounded_blocks(small):
+    """Rows of more than one 16 MB block (38 of 9,126 pairs or 7 of 45,630, the last block a ragged one) are the single
+    rows, and the context keeps no more than the block."""
+    import torch
+
+    from haseongpu_b200 import DeviceMesh
+
+    mesh, sa, se, _ = small
+    assert mesh.numberOfPrisms == 9126
+    with DeviceMesh(mesh, sa, se) as ctx:
+        for reflections, count in ((False, 83), (True, 17)):
+            one = ctx.proposal_features(5, 1, useReflections=reflections)
+            free = torch.cuda.mem_get_info()[0]
+            many = ctx.proposal_features(5, count, useReflections=reflections)
+            assert free - torch.cuda.mem_get_info()[0] < 24 << 20
+            np.testing.assert_array_equal(many[0], one[0])
+            for i in sorted({6, 7, 13, min(37, count - 1), min(38, count - 1), count - 1}):
+                np.testing.assert_array_equal(many[i], ctx.proposal_features(5 + i, 1, useReflections=reflections)[0])
