@@ -117,7 +117,7 @@ struct ImportanceLaunch {
     uint32_t firstSample, rows, slices, nW;
     const float2* line;  // [T][phases layers]: meshTablesKernel
     float* lnw;   // [rows][nW]
-    const uint32_t* rowList;  // rows to compute (blockIdx.y indexes it), or null: rows 0 .. rows - 1
+    const uint32_t* rowList;  // rows to compute (y0 + blockIdx.y indexes it), or null: rows 0 .. rows - 1
     const uint8_t* rowFlag;   // batched media: only rows with rowFlag[flagBase + row] set are computed (or null)
     uint32_t flagBase;
     unsigned long long* crossings;  // counting launches only: total walk crossings
@@ -126,6 +126,7 @@ struct ImportanceLaunch {
     const uint32_t* cand;
     uint32_t K;
     uint32_t divLm, divLs;  // floor(x / layers) = (x * divLm) >> divLs
+    uint32_t y0;            // blockIdx.y = 0 is this row (a grid has at most 65,535 of them)
 };
 
 // The lines' table (TableJob::line): per triangle the gain along z in the unfolded
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
     constexpr int kRoundBits = 0x4B400000;
     const uint32_t tIdx = blockIdx.x * kTeams + threadIdx.x / TL;  // triangle (or candidate) of the team
     const uint32_t li = threadIdx.x % TL;
-    const uint32_t row0 = L.rowList ? L.rowList[blockIdx.y] : blockIdx.y;
+    const uint32_t row0 = L.rowList ? L.rowList[L.y0 + blockIdx.y] : L.y0 + blockIdx.y;
     const uint32_t strideL = L.cand ? L.K : m.T;            // entries per layer of a slice
     unsigned long long counted = 0;
     if (tIdx < strideL && !(L.rowFlag && !L.rowFlag[L.flagBase + row0])) {
@@ -375,6 +376,8 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
     }
 }
 
+constexpr uint32_t kMaxGridY = 65535;  // blocks of a grid in y
+
 // The importance walks of `rows` sample rows (il.rowList: that many listed
 // rows).  A point's lines -- its requested levels x slices x layers -- fill the
 // narrowest team that holds them with at most 4 per lane, in as few chunks of
@@ -393,28 +396,33 @@ cudaError_t launchImportance(ImportanceLaunch il, uint32_t meshLayers, uint32_t 
     const uint32_t lpl = uint32_t((lines + tl * chunks - 1) / (tl * chunks));
 #define HASE_TEAM(TL, LPL)                                                            \
     {                                                                                 \
-        const dim3 grid((nTri + 256 / TL - 1) / (256 / TL), gridRows);                \
+        const dim3 grid((nTri + 256 / TL - 1) / (256 / TL), gridY);                   \
         importanceTeamKernel<TL, LPL><<<grid, 256, 0, stream>>>(il);                  \
     }
-    if (count) {
-        const dim3 grid((nTri + 7) / 8, gridRows);
-        importanceTeamKernel<32, 3, true><<<grid, 256, 0, stream>>>(il);
-    } else if (tl == 4) {
-        switch (lpl) {
-            case 1: HASE_TEAM(4, 1) break;
-            case 2: HASE_TEAM(4, 2) break;
-            case 3: HASE_TEAM(4, 3) break;
-            default: HASE_TEAM(4, 4) break;
+    for (il.y0 = 0; il.y0 < gridRows; il.y0 += kMaxGridY) {
+        const uint32_t gridY = std::min(gridRows - il.y0, kMaxGridY);
+        if (count) {
+            const dim3 grid((nTri + 7) / 8, gridY);
+            importanceTeamKernel<32, 3, true><<<grid, 256, 0, stream>>>(il);
+        } else if (tl == 4) {
+            switch (lpl) {
+                case 1: HASE_TEAM(4, 1) break;
+                case 2: HASE_TEAM(4, 2) break;
+                case 3: HASE_TEAM(4, 3) break;
+                default: HASE_TEAM(4, 4) break;
+            }
+        } else if (tl == 8) {
+            if (lpl <= 3) HASE_TEAM(8, 3) else HASE_TEAM(8, 4)
+        } else if (tl == 16) {
+            if (lpl <= 3) HASE_TEAM(16, 3) else HASE_TEAM(16, 4)
+        } else {
+            if (lpl <= 3) HASE_TEAM(32, 3) else HASE_TEAM(32, 4)
         }
-    } else if (tl == 8) {
-        if (lpl <= 3) HASE_TEAM(8, 3) else HASE_TEAM(8, 4)
-    } else if (tl == 16) {
-        if (lpl <= 3) HASE_TEAM(16, 3) else HASE_TEAM(16, 4)
-    } else {
-        if (lpl <= 3) HASE_TEAM(32, 3) else HASE_TEAM(32, 4)
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
 #undef HASE_TEAM
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 bool validImportanceLayers(uint32_t layers) {
@@ -1673,7 +1681,7 @@ __global__ void __launch_bounds__(256) gridWeightKernel(const ProposalLaunch P) 
 static cudaError_t launchGridWeights(const ProposalLaunch& gl, cudaStream_t s) {
     const uint32_t width = gl.V.cand ? gl.V.m.layers * gl.V.K : gl.V.m.P;
     if (width == 0 || gl.rows == 0) return cudaSuccess;
-    const dim3 grid((width + 255) / 256, std::min<uint32_t>(gl.rows, 65535u));
+    const dim3 grid((width + 255) / 256, std::min<uint32_t>(gl.rows, kMaxGridY));
     gridWeightKernel<<<grid, 256, 0, s>>>(gl);
     return cudaGetLastError();
 }
@@ -2954,7 +2962,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
         il.cand = local ? c->candTri.p : nullptr;
         il.K = K;
         auto launchImportanceRows = [&](uint32_t nLaunchRows) {
-            launchImportance(il, c->layers, c->T, c->Np, nLaunchRows, c->stream);
+            return launchImportance(il, c->layers, c->T, c->Np, nLaunchRows, c->stream);
         };
         if (la) {
             pv.firstSample = firstSample;
@@ -2974,7 +2982,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
             const ProposalLaunch gl{pv, nullptr, nullptr, c->lnw.p, nullptr, nullptr, nRows, nullptr};
             HASE_CUDA(launchGridWeights(gl, c->stream));
         } else {
-            launchImportanceRows(nRows);
+            HASE_CUDA(launchImportanceRows(nRows));
         }
         if (farPrior) {  // the far prior's cell prefixes of the chunk's rows
             FarRowLaunch fl{c->cellXY.p, c->cellMass.p, c->gCell.p, c->gTab.p, c->candTri.p, c->farCells, slices,
@@ -3104,7 +3112,7 @@ static hase_status calcCore(hase_context* c, const hase_experiment_desc* ex, con
                                               c->stream));
                     HASE_CUDA(cudaEventRecord(c->ev[2], c->stream));
                     il.rowList = c->rowList.p;
-                    launchImportanceRows(nf);
+                    HASE_CUDA(launchImportanceRows(nf));
                     il.rowList = nullptr;
                     HASE_CUDA(cudaGetLastError());
                     HASE_CUDA(cudaEventRecord(c->ev[3], c->stream));
@@ -4323,8 +4331,8 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
     // the views' gain grids are built on each context's own stream: finished
     // before the batch's stream reads them
     for (uint32_t i = 0; i < count; ++i) HASE_CUDA(cudaStreamSynchronize(media[i].c->stream));
-    for (uint32_t i = 0; i < count; i += 65535) {
-        const uint32_t n = std::min(count - i, 65535u);
+    for (uint32_t i = 0; i < count; i += kMaxGridY) {
+        const uint32_t n = std::min(count - i, kMaxGridY);
         meshTablesKernel<<<dim3((maxT + 127) / 128, n), 128, 0, b->stream>>>(b->tableJobs.p + i, TableJob{});
         HASE_CUDA(cudaGetLastError());
     }

@@ -82,3 +82,37 @@ def test_grouped_levels_give_the_single_rows(oracle, levels, reflections):
         big = ref > 1e-6
         rel = np.abs(every[s][big] / ref[big] - 1.0)
         assert np.quantile(rel, 0.999) < 1e-5 and rel.max() < 5e-4
+
+
+def _square(n, rng=None):
+    """n x n points on a square, two triangles per cell, one layer."""
+    from haseongpu_b200 import PrismMesh
+
+    x = np.linspace(-1.0, 1.0, n)
+    pts = np.column_stack([np.tile(x, n), np.repeat(x, n)])
+    i = (np.arange(n - 1)[:, None] * n + np.arange(n - 1)[None]).ravel()
+    tri = np.concatenate([np.column_stack([i, i + 1, i + n]), np.column_stack([i + 1, i + n + 1, i + n])]).astype(np.uint32)
+    beta = 0.1 + 0.2 * np.cos(np.arange(tri.shape[0]))**2
+    return PrismMesh(points=pts, triangles=tri, numberOfLevels=2, thickness=0.1, betaVolume=beta, nTot=1.38e20,
+                     crystalTFluo=1e-3)
+
+
+def test_more_rows_than_a_grid_has_in_y():
+    """66,049 points in one workspace: a grid has 65,535 blocks in y, so the rows past them are another launch; the same
+    weights and estimates as in two ranges of fewer rows."""
+    from haseongpu_b200 import DeviceMesh
+
+    mesh = _square(257)
+    Np, half = mesh.numberOfPoints, 40_000
+    assert Np > 65_535
+    kw = dict(minRays=32, rngSeed=3, workspaceBytes=64 << 30)
+    with DeviceMesh(mesh, [1.1e-21], [2.2e-20]) as ctx:
+        ctx.set_local_proposal(2)
+        every = ctx.importance_weights(0, 2 * Np, False)
+        np.testing.assert_array_equal(every[:half], ctx.importance_weights(0, half, False))
+        np.testing.assert_array_equal(every[2 * Np - half:], ctx.importance_weights(2 * Np - half, half, False))
+        whole = ctx.calc_phi_ase(maxSample=Np - 1, **kw)
+        parts = [ctx.calc_phi_ase(minSample=a, maxSample=b, **kw) for a, b in ((0, half - 1), (half, Np - 1))]
+    assert np.all(np.isfinite(every)) and np.all(every.max(axis=1) == 1.0)
+    for k in ("phiAse", "relativeStandardError", "totalRays", "droppedRays"):
+        np.testing.assert_array_equal(getattr(whole, k), np.concatenate([getattr(p, k) for p in parts]))
