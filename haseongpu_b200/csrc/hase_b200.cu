@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <chrono>
 #include <limits>
 #include <cmath>
@@ -225,7 +226,12 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
         const float area = __ldg(&m.geo[2 * t + 1].z);
         const float dx = c.x - S.x, dy = c.y - S.y;
         const float D2 = sqrtf(fmaf(dx, dx, dy * dy));
-        const float inv2 = 1.0f / D2;
+        // The line's table entries come from sOut * inv, so both stay finite: a
+        // prism straight above or below the sample (in FP32, a centroid on a
+        // vertex) has a line of no length in the plane, and a sample at a
+        // coordinate that is not finite has no line (NaN weights).
+        const bool finite = D2 <= FLT_MAX;
+        const float inv2 = finite && D2 > 0.0f ? 1.0f / D2 : 0.0f;
         const float ux = dx * inv2, uy = dy * inv2;
         const size_t strideJ = size_t(strideL) * m.layers;
         const uint32_t stride = linePhases(L.slices) * m.layers;
@@ -285,7 +291,7 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
             uint32_t w = firstWindow;
             float4 wa = __ldg(m.win + w), wb = __ldg(m.win + w + 1);
             uint32_t columns = 0;
-            float sc = D2;
+            float sc = finite ? D2 : 0.0f;
             bool done = false;
             for (int step = 0; step < kMaxSteps && !done; ++step) {
                 const uint32_t tk = w >> 2;
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
                         // the bounce happens at the target itself, in the final triangle
                         if (j > 0 && ls == (j == 1 || j == 4 ? 0 : layers))
                             ln += __logf(reflectFactor(m, tk, j == 1 || j == 4 ? 0 : 1, dz * rsqrtf(D3sq)));
-                        v = __logf(beta * area * m.h / D3sq) + acc[g] * (sqrtf(D3sq) / a) + ln;
+                        v = finite ? __logf(beta * area * m.h / D3sq) + acc[g] * (sqrtf(D3sq) / a) + ln : NAN;
                     }
                 }
                 L.lnw[size_t(row0 + uint32_t(ls - ls0) * m.Np) * L.nW + size_t(j) * strideJ + size_t(l) * strideL + tIdx] = v;

@@ -116,3 +116,48 @@ def test_more_rows_than_a_grid_has_in_y():
     assert np.all(np.isfinite(every)) and np.all(every.max(axis=1) == 1.0)
     for k in ("phiAse", "relativeStandardError", "totalRays", "droppedRays"):
         np.testing.assert_array_equal(getattr(whole, k), np.concatenate([getattr(p, k) for p in parts]))
+
+
+@pytest.mark.parametrize("reflections", [False, True])
+def test_lines_of_no_length_and_no_place(oracle, reflections):
+    """A triangle smaller than an FP32 spacing has its centroid on its own vertices: its prisms are straight above and
+    below those samples, and their weights are the oracle's (3e-4: positions rounded by up to 4e-6, 0.1 apart, squared).  A
+    point that no triangle uses and that is nowhere (NaN, inf) has no weights and leaves the other samples' alone."""
+    from haseongpu_b200 import DeviceMesh
+
+    mesh = _square(5)
+    mesh.points = mesh.points + 100.0
+    a, b, c = mesh.triangles[7].astype(int)
+    A, B, C = mesh.points[a], mesh.points[b], mesh.points[c]
+    p1, p2 = (A + 1e-6 * (x * (B - A) + y * (C - A)) for x, y in ((0.6, 0.2), (0.2, 0.6)))
+    i, j = len(mesh.points), len(mesh.points) + 1
+    mesh.points = np.vstack([mesh.points, p1, p2])
+    more = np.array([[a, i, j], [a, b, i], [b, c, i], [i, c, j], [a, j, c]], np.uint32)
+    mesh.triangles = np.vstack([mesh.triangles[:7], mesh.triangles[8:], more])
+    T = mesh.triangles.shape[0]
+    layers = 4
+    mesh.numberOfLevels = layers + 1
+    mesh.betaVolume = np.random.default_rng(3).uniform(0.05, 0.3, T * layers)
+    mesh.reflectivities = np.tile([0.3, 0.9], (T, 1))
+    mesh.refractiveIndices = np.array([1.83, 1.0, 1.83, 1.0])
+    tiny = T - 5
+    cen = mesh.points[mesh.triangles[tiny]].astype(np.float32)
+    assert np.all(cen == np.float32(mesh.points[a]))
+    spectrum, slices = ([1.1e-21], [2.2e-20]), 5 if reflections else 1
+    Np = mesh.numberOfPoints
+    with DeviceMesh(mesh, *spectrum) as ctx:
+        for pt in (a, i, j):
+            for level in (0, 2, layers):
+                w = ctx.importance_weights(level * Np + pt, 1, reflections)[0].astype(np.float64)
+                ref = np.asarray(oracle.importance(mesh, spectrum, level * Np + pt, slices=slices), float).ravel()
+                at = (np.arange(slices * layers) * T + tiny)
+                assert np.all(np.isfinite(w))
+                np.testing.assert_allclose(w[at] / w.max(), ref[at] / ref.max(), rtol=3e-4)
+        plain = ctx.importance_weights(0, layers + 1, reflections)
+    for nowhere in (np.nan, np.inf):
+        mesh.points = np.vstack([mesh.points[:Np], [[nowhere, 0.0]]])
+        with DeviceMesh(mesh, *spectrum) as ctx:
+            w = ctx.importance_weights(Np, 1, reflections)[0]
+            assert not np.any(np.isfinite(w) & (w > 0))
+            if np.isnan(nowhere):
+                np.testing.assert_array_equal(ctx.importance_weights(0, layers + 1, reflections), plain)
