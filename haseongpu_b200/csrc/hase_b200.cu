@@ -116,7 +116,7 @@ void invariantDivisor(uint32_t d, uint32_t& mul, uint32_t& shift) {
 struct ImportanceLaunch {
     MeshView m;
     uint32_t firstSample, rows, slices, nW;
-    const float2* line;  // [T][phases layers]: meshTablesKernel
+    const float2* line;  // [T][lineStride]: meshTablesKernel
     float* lnw;   // [rows][nW]
     const uint32_t* rowList;  // rows to compute (y0 + blockIdx.y indexes it), or null: rows 0 .. rows - 1
     const uint8_t* rowFlag;   // batched media: only rows with rowFlag[flagBase + row] set are computed (or null)
@@ -135,20 +135,28 @@ struct ImportanceLaunch {
 // sequence down, up, down (phases x layers entries, i falling along a line's
 // way: phase 0 is a line moving down in layer i, phase 1 one moving up in
 // layer 2 layers - 1 - i, phase 2 down again) and holds (F, g): g of the layer's
-// prism (beta A - B, -claddingAbsorption in cladding) and F = the integral of g
-// over the sequence up to the middle of the entry, in level units, summed in
-// FP64 and centred so that its FP32 rounding is small.  A line's integral over
-// any stretch of a triangle is then a difference of two F + g (position -
-// middle), whatever the number of levels and reflections in between.
+// prism (beta A - B, -claddingAbsorption in cladding) minus the triangle's mean
+// over its layers, and F = the integral of that over the sequence up to the
+// middle of the entry, in level units, summed in FP64; the mean is the last
+// entry.  A line's integral over any stretch of a triangle is then the mean
+// times its levels and a difference of two F + g (position - middle), whatever
+// the number of levels and reflections in between.  Without the mean F spans a
+// few levels of the field's variation in z instead of the whole way's gain, and
+// its FP32 rounding stays below that of the lines' own sums (256 samples of a
+// 5,046-triangle x 19-layer disc, weights 10.2 ms without the mean, 11.0 with; in
+// a medium with a gain of e^50 over its height the rms error of ln w 5e-6 and 1e-6).
 // Without reflections a line stays in phase 0 or 1 (phases = 2).
 struct TableJob {
     const float* gainBeta;  // [layers][T], NaN in cladding
     float A, B, cladAbs;
     uint32_t T, layers, phases;
-    float2* line;           // [T][phases layers] or null
+    float2* line;           // [T][lineStride] or null
     float* walk;            // [T][layers]: the ray walk's table (MeshView::walkTab)
     int walkGain;           // its values: g, or beta
 };
+
+__host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slices == 1 ? 2u : 3u; }
+__host__ __device__ constexpr uint32_t lineStride(uint32_t phases, uint32_t layers) { return phases * layers + 1u; }
 
 // A medium's tables for one solve, one thread per triangle; jobs: one medium per
 // blockIdx.y (a batch), or null: `one`.
@@ -166,19 +174,19 @@ __global__ void meshTablesKernel(const TableJob* jobs, TableJob one) {
         total += double((b == b) ? g : -absorb);
     }
     if (!J.line) return;
-    float2* out = J.line + size_t(t) * J.phases * J.layers;
-    double F = -0.5 * double(J.phases) * total;
+    float2* out = J.line + size_t(t) * lineStride(J.phases, J.layers);
+    const float mean = float(total / double(J.layers));
+    double F = 0.0;
     for (uint32_t ph = 0, i = 0; ph < J.phases; ++ph)
         for (uint32_t r = 0; r < J.layers; ++r, ++i) {
             const uint32_t l = ph & 1u ? J.layers - 1u - r : r;
             const float b = __ldg(J.gainBeta + size_t(l) * J.T + t);
-            const float g = (b == b) ? fmaf(b, J.A, -J.B) : -absorb;
-            out[i] = make_float2(float(F + 0.5 * double(g)), g);
-            F += double(g);
+            const double g = double((b == b) ? fmaf(b, J.A, -J.B) : -absorb) - double(mean);
+            out[i] = make_float2(float(F + 0.5 * g), float(g));
+            F += g;
         }
+    out[J.phases * J.layers] = make_float2(mean, 0.0f);
 }
-
-__host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slices == 1 ? 2u : 3u; }
 
 // Line-team importance kernel: a team of TL lanes per (sample point,
 // triangle t).  Every line from the centre of a prism (t, l) to an image of a
@@ -193,7 +201,7 @@ __host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slic
 // table entry is n + base.  Per triangle and line: the entry and the position
 // in it at the exit (one FFMA, one rounding by 1.5 2^23, two adds), one table
 // load at the entry and one at the exit, and five operations for the
-// integral.  Stepping through the levels one by one cost a loop per line that
+// integral; the triangles' mean g, the same for all lines, is summed once.  Stepping through the levels one by one cost a loop per line that
 // the warp ran as often as its steepest line needed (216 warp instructions per
 // triangle for 96 lines).
 // A bounce is only an event (the branch) for its factor, which a line beyond
@@ -204,7 +212,7 @@ __host__ __device__ constexpr uint32_t linePhases(uint32_t slices) { return slic
 // COUNT: also add the walk's crossings (triangle segments plus level planes
 // and reflections, per line) to *L.crossings.
 template <int TL, int LPL, bool COUNT = false>
-__global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) {
+__global__ void __launch_bounds__(256, LPL <= 3 ? 3 : 2) importanceTeamKernel(ImportanceLaunch L) {
     static_assert(TL >= 1 && TL <= 32 && (32 % TL) == 0, "a team is a power-of-two part of a warp");
     const MeshView& m = L.m;
     constexpr uint32_t kTeams = 256 / TL;
@@ -225,16 +233,17 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
         const float2 c = __ldg(m.centroid + t);
         const float area = __ldg(&m.geo[2 * t + 1].z);
         const float dx = c.x - S.x, dy = c.y - S.y;
-        const float D2 = sqrtf(fmaf(dx, dx, dy * dy));
         // The line's table entries come from sOut * inv, so both stay finite: a
         // prism straight above or below the sample (in FP32, a centroid on a
-        // vertex) has a line of no length in the plane, and a sample at a
-        // coordinate that is not finite has no line (NaN weights).
-        const bool finite = D2 <= FLT_MAX;
-        const float inv2 = finite && D2 > 0.0f ? 1.0f / D2 : 0.0f;
+        // vertex) has a line of next to no length in the plane, and a sample at a
+        // coordinate that is not finite has none (NaN weights).
+        const float dist = sqrtf(fmaf(dx, dx, dy * dy));
+        const bool finite = dist <= FLT_MAX;
+        const float D2 = finite ? fmaxf(dist, 1e-18f) : 1e-18f;
+        const float inv2 = 1.0f / D2;
         const float ux = dx * inv2, uy = dy * inv2;
         const size_t strideJ = size_t(strideL) * m.layers;
-        const uint32_t stride = linePhases(L.slices) * m.layers;
+        const uint32_t stride = lineStride(linePhases(L.slices), m.layers);
         // rows of the point: row0, row0 + Np, ... (listed and flagged rows one by one)
         const uint32_t levels = L.rowList || L.rowFlag ? 1u : 1u + (L.rows - 1u - row0) / m.Np;
         const uint32_t nLines = levels * L.slices * m.layers;
@@ -291,7 +300,7 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
             uint32_t w = firstWindow;
             float4 wa = __ldg(m.win + w), wb = __ldg(m.win + w + 1);
             uint32_t columns = 0;
-            float sc = finite ? D2 : 0.0f;
+            float sc = D2, mean = 0.0f;  // mean: the triangles' mean g over the segment
             bool done = false;
             for (int step = 0; step < kMaxSteps && !done; ++step) {
                 const uint32_t tk = w >> 2;
@@ -307,6 +316,7 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
                 float sOut = fminf(qm, sc);
                 done = !(sOut > m.tolEnd);
                 sOut = done ? 0.0f : sOut;
+                mean = fmaf(__ldg(&col[stride - 1].x), sc - sOut, mean);
                 if (COUNT) ++columns;
                 float n[LPL], fo[LPL];
                 int bits[LPL];
@@ -369,7 +379,8 @@ __global__ void __launch_bounds__(256) importanceTeamKernel(ImportanceLaunch L) 
                         // the bounce happens at the target itself, in the final triangle
                         if (j > 0 && ls == (j == 1 || j == 4 ? 0 : layers))
                             ln += __logf(reflectFactor(m, tk, j == 1 || j == 4 ? 0 : 1, dz * rsqrtf(D3sq)));
-                        v = finite ? __logf(beta * area * m.h / D3sq) + acc[g] * (sqrtf(D3sq) / a) + ln : NAN;
+                        const float gain = fmaf(mean, inv[g], acc[g]) * (sqrtf(D3sq) / a);
+                        v = finite ? __logf(beta * area * m.h / D3sq) + gain + ln : NAN;
                     }
                 }
                 L.lnw[size_t(row0 + uint32_t(ls - ls0) * m.Np) * L.nW + size_t(j) * strideJ + size_t(l) * strideL + tIdx] = v;
@@ -2461,7 +2472,7 @@ TableJob tableJob(const hase_context* c, double A, double B, uint32_t slices, bo
 }
 
 hase_status buildTables(hase_context* c, double A, double B, uint32_t slices, bool walkGain) {
-    if (slices) HASE_CUDA(c->line.ensure(size_t(c->P) * linePhases(slices)));
+    if (slices) HASE_CUDA(c->line.ensure(size_t(c->T) * lineStride(linePhases(slices), c->layers)));
     meshTablesKernel<<<(c->T + 127) / 128, 128, 0, c->stream>>>(
         nullptr, tableJob(c, A, B, slices, walkGain, c->line.p, c->walkTab.p));
     HASE_CUDA(cudaGetLastError());
@@ -4283,7 +4294,7 @@ hase_status batchCore(hase_batch* b, const hase_batch_instance* in, uint32_t cou
         const hase_context* c = media[i].c;
         lineAt[i] = lineEntries;
         walkAt[i] = walkEntries;
-        lineEntries += walksOf(i) ? size_t(c->P) * linePhases(slices) : 0;
+        lineEntries += walksOf(i) ? size_t(c->T) * lineStride(linePhases(slices), c->layers) : 0;
         walkEntries += c->P;
         maxT = std::max(maxT, c->T);
     }
