@@ -192,11 +192,8 @@ __device__ __forceinline__ float initRay(Ray& r, uint32_t t, int layer, float dx
     const float h = m.h;
     if (dz == 0.0f) dz = 1e-6f * h;  // a ray inside a level plane: nudge it off the plane
     const float D2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    // 1 / D to its last bit or two: the approximation and one Newton step (a
-    // rounded square root and a rounded division took three times the instructions)
-    const float i0 = rsqrtf(D2);
-    const float inv = fmaf(0.5f * i0, fmaf(-D2 * i0, i0, 1.0f), i0);
-    const float D = D2 * inv;
+    const float D = sqrtf(D2);
+    const float inv = 1.0f / D;
     r.row = layer;
     r.reflLeft = expectedReflections(slice);
     r.s = D;
