@@ -676,13 +676,10 @@ __device__ __forceinline__ float farSliceFactor(const FarSlices& S, uint32_t j, 
     return j == 1 ? rb : (j == 2 ? rt : rb * rt);
 }
 
-// One term of the far prior: R_j m e^Ghat / d^2, Ghat = gmean d, from one
-// reciprocal square root (a square root and a division per layer of every scan
-// were a tenth of the local proposal's row kernel).
+// One term of the far prior: R_j m e^Ghat / d^2, Ghat = gmean d.
 __device__ __forceinline__ float farTerm(float prior, float mass, float d2, float gmean) {
-    const float r = rsqrtf(d2);
-    const float G = fminf(fmaxf(gmean * (d2 * r), -10.0f), 30.0f);
-    return prior * mass * __expf(G) * (r * r);
+    const float G = fminf(fmaxf(gmean * sqrtf(d2), -10.0f), 30.0f);
+    return __fdividef(prior * mass * __expf(G), d2);
 }
 
 // The far prior's mean g along the way, (g_cl + g_s + 6 g_mid) / 8.
