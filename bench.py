@@ -390,7 +390,7 @@ def measure_importance(args, local, rank=0, world=1, nested=False):
                        "rays_per_sample": [w.minRays, w.maxRays], "threshold": w.threshold,
                        "adaptive_steps": w.adaptiveSteps, "parallelism": f"sample batches x{world}",
                        "l2": "flushed (256 MiB write) before every timed step; per-step weights > L2",
-                       "ray_kernel": {"variant": tuned.name, "rays_per_item": 32 * tuned.raysPerThread,
+                       "ray_kernel": {"variant": tuned.name, "rays_per_item": 32 * tuned.raysPerThread or "automatic",
                                       "autotuned_ms": tuned.milliseconds},
                        "importance_kernel": {"layers_per_thread": tuned.importanceLayers,
                                              "autotuned_ms": tuned.importanceMilliseconds}},
@@ -750,7 +750,7 @@ def measure_media(args, local, steps, warmup):
                    "wavelengths": [m.wavelengths for m in w.media], "rays_per_sample": [w.minRays, w.maxRays],
                    "threshold": w.threshold, "adaptive_steps": w.adaptiveSteps,
                    "l2": "flushed (256 MiB write) before every timed step",
-                   "ray_kernel": {"variant": tune.name, "rays_per_lane": tune.raysPerThread,
+                   "ray_kernel": {"variant": tune.name, "rays_per_lane": tune.raysPerThread or "automatic",
                                   "autotuned_over": len(tune.table)}},
         "breakdown_ms_per_step": {"proposal_and_mixture": L["imp_ms"] / steps,
                                   "map_ray_finalise_passes": L["ray_ms"] / steps,
@@ -1159,7 +1159,7 @@ def run_learned(args):
             "dtype": "f32 geometry, f64 sums, bf16 proposal network (f32 accumulation)",
             "data": "synthetic (seeded gain media and pump fields, no dataset)",
             "config": learned_config(w, mesh, world),
-            "ray_kernel": {"variant": tuned.name, "rays_per_lane": tuned.raysPerThread,
+            "ray_kernel": {"variant": tuned.name, "rays_per_lane": tuned.raysPerThread or "automatic",
                            "importance_layers": tuned.importanceLayers, "autotuned_over": len(tuned.table)},
             "time_to_threshold_ms": ms_l / args.steps,
             "plain_is": {"value": solved_all / (ms_p * 1e-3), "unit": "samples/s", "ms_per_step": ms_p / args.steps,

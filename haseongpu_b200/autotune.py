@@ -2,7 +2,8 @@
 
 Sweeps every launch shape libhase_b200 compiles (block size, idle lanes that
 trigger a batched refill, occupancy target; ``hase_ray_kernel_variant_name``)
-and the work-item size (rays per lane of a work item) on a short, fixed-ray
+and the work-item size (rays per lane of a work item; 0: the size the library
+chooses from the rays of each pass) on a short, fixed-ray
 solve of the caller's own workload, timing only the ray kernel with the CUDA
 events the library records, and returns the fastest pair.  Results are
 cached per process by (device, mesh size, reflections, wavelengths).
@@ -14,7 +15,7 @@ from dataclasses import dataclass
 
 from . import _native as N
 
-RAYS_PER_LANE = (16, 32, 64, 128)  # work items of 512 .. 4096 rays
+RAYS_PER_LANE = (0, 16, 32, 64, 128)  # the library's choice from each pass's rays, or work items of 512 .. 4096 rays
 
 _cache: dict = {}
 
@@ -68,15 +69,10 @@ def autotune(ctx, *, firstSample: int, samples: int, rays: int, useReflections: 
             table.append({"variant": v, "name": name, "raysPerThread": rpt, "ray_ms": t})
             if best is None or t < best[2]:
                 best = (v, rpt, t)
-    imp = []
-    for layers in (0,):  # the line-team kernel: the one importance kernel there is
-        t = min(ctx.calc_phi_ase(minRays=1, maxRays=1, useReflections=useReflections, monochromatic=monochromatic,
-                                 nearFieldSampling=nearFieldSampling, rngSeed=3, minSample=firstSample,
-                                 maxSample=firstSample + samples - 1, importanceLayers=layers).importanceMilliseconds
-                for _ in range(repeats))
-        imp.append((t, layers))
-        table.append({"importanceLayers": layers, "importance_ms": t})
-    result = TuneResult(best[0], best[1], names[best[0]], best[2], table, min(imp)[1], min(imp)[0])
+    imp = min(ctx.calc_phi_ase(minRays=1, maxRays=1, useReflections=useReflections, monochromatic=monochromatic,
+                               nearFieldSampling=nearFieldSampling, rngSeed=3, minSample=firstSample,
+                               maxSample=firstSample + samples - 1).importanceMilliseconds for _ in range(repeats))
+    result = TuneResult(best[0], best[1], names[best[0]], best[2], table, 0, imp)
     _cache[key] = result
     return result
 
