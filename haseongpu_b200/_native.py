@@ -44,6 +44,7 @@ EXPORTED_SYMBOLS = (
     "hase_importance_crossings",
     "hase_ray_map",
     "hase_mesh_tables",
+    "hase_mesh_windows",
     "hase_trace_rays",
     "hase_philox",
     "hase_probe_l2_bandwidth",

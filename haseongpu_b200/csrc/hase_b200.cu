@@ -3860,6 +3860,16 @@ hase_status hase_mesh_tables(const hase_mesh_desc* d, float* tri, float* walk) {
     return HASE_OK;
 }
 
+hase_status hase_mesh_windows(const hase_mesh_desc* d, float* windows) {
+    if (!d || !d->points || !d->triangles || !windows || d->numberOfTriangles == 0)
+        return fail(HASE_INVALID_ARGUMENT, "mesh points, triangles and an output array are required");
+    HostTables ht;
+    double extent = 0.0;
+    HASE_TRY(buildHostTables(d, ht, extent));
+    std::memcpy(windows, ht.win.data(), ht.win.size() * sizeof(float4));
+    return HASE_OK;
+}
+
 hase_status hase_trace_rays(hase_context* c, uint32_t n, const float* start, const uint32_t* tri,
                             const uint32_t* level, const uint32_t* sample, const uint32_t* slice, uint32_t wavelength,
                             float* lnGain, float* distance, uint32_t* dropped) {

@@ -214,6 +214,14 @@ hase_status hase_importance_crossings(hase_context* ctx, uint32_t firstSample, u
  * either may be NULL. */
 hase_status hase_mesh_tables(const hase_mesh_desc* mesh, float* tri, float* walk);
 
+/* The edge windows that the walks read, built on the host (no device needed):
+ * windows[numberOfTriangles][4][4], a triangle's edges in the slots e0 e1 e2
+ * e0, each (nx, ny, c, code).  The two slots from the window's first one are
+ * the edges other than the one the walk entered through (entered through e0:
+ * slots 1, 2; e1: 2, 3; e2: 0, 1).  code (int bits) is the window on the other
+ * side, 4 neighbour + first slot.  A mesh-boundary edge is (0, 0, 1, 0). */
+hase_status hase_mesh_windows(const hase_mesh_desc* mesh, float* windows);
+
 /* Ray->prism map of `rows` weight rows of length n: q[row][n] (quantised
  * weights), offsets[row][n+1] (exclusive ray offsets), Q[row]. */
 hase_status hase_ray_map(uint32_t rows, uint32_t n, const float* weights, uint32_t rays, const uint32_t* phases,

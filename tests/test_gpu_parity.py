@@ -88,27 +88,57 @@ def test_trace_with_reflections_matches_oracle(oracle):
     assert np.quantile(err, 0.999) < 1e-5 and err.max() < 5e-4, (err.max(), np.quantile(err, 0.999))
 
 
+def _lines_crossings(mesh, s, slices):
+    """Crossings of sample s's lines in FP64: the triangles on the way from each prism's centroid to the sample point
+    plus the level planes on the way to its image, over the prisms with a source."""
+    p, tri = mesh.points, mesh.triangles.astype(int)
+    T, layers = tri.shape[0], mesh.numberOfLevels - 1
+    edges = {}
+    for t in range(T):
+        for e in range(3):
+            edges.setdefault(tuple(sorted((tri[t, e], tri[t, (e + 1) % 3]))), []).append(t)
+    S, ls = p[s % mesh.numberOfPoints], s // mesh.numberOfPoints
+    cen = p[tri].mean(1)
+
+    def side(q, r, x):
+        return (r[..., 0] - q[..., 0]) * (x[..., 1] - q[..., 1]) - (r[..., 1] - q[..., 1]) * (x[..., 0] - q[..., 0])
+
+    columns = np.ones(T)  # the line's own triangle, then one for every inner edge it crosses
+    for (a, b), ts in edges.items():
+        if len(ts) == 2 and s % mesh.numberOfPoints not in (a, b):
+            A, B = p[a], p[b]
+            columns += (side(A, B, cen) * side(A, B, S) < 0) & (side(cen, S, A) * side(cen, S, B) < 0)
+    images = [ls, -ls, 2 * layers - ls, ls - 2 * layers, ls + 2 * layers][:slices]
+    source = (np.asarray(mesh.betaVolume).reshape(layers, T) > 0).astype(float)
+    return sum((source[l] * (columns + np.floor(abs(l + 0.5 - k)))).sum() for k in images for l in range(layers))
+
+
 @pytest.mark.parametrize("workload", ["disc_small", "disc_poly"])
-def test_importance_kernels_give_identical_estimates(workload):
-    """The line-team kernel (importanceLayers 0) and the layer-group kernel
-    (2, 4, 8 layers per thread) run the same per-line arithmetic: identical
-    weights, hence identical ray maps and bit-identical estimates; and the
-    crossing count of the walks is positive and reproducible."""
+def test_importance_layers_and_crossings(workload):
+    """importanceLayers takes 0, 2, 4 and 8, which the library no longer tells apart, and refuses the rest.  The
+    crossing count of the importance walks is that of straight lines in FP64 (1e-3: lines through a vertex)."""
     from haseongpu_b200 import configs
 
     w = configs.WORKLOADS[workload]()
     sa, se = w.spectra.resampled(w.monochromatic)
     kw = dict(minRays=3000, useReflections=w.useReflections, monochromatic=w.monochromatic, rngSeed=5,
               minSample=100, maxSample=131)
+    picks = [100, w.mesh.numberOfPoints * 4 + 31]
     with _ctx(w.mesh, sa, se) as ctx:
         runs = [ctx.calc_phi_ase(importanceLayers=g, **kw) for g in (0, 2, 4, 8)]
+        for g in (1, 3, 16):
+            with pytest.raises(RuntimeError, match="importanceLayers"):
+                ctx.calc_phi_ase(importanceLayers=g, **kw)
         n1 = ctx.importance_crossings(100, 32, w.useReflections)
         n2 = ctx.importance_crossings(100, 32, w.useReflections)
+        counts = [ctx.importance_crossings(s, 1, w.useReflections) for s in picks]
     for r in runs[1:]:
         np.testing.assert_array_equal(r.phiAse, runs[0].phiAse)
         np.testing.assert_array_equal(r.relativeStandardError, runs[0].relativeStandardError)
     lines = 32 * (5 if w.useReflections else 1) * w.mesh.numberOfPrisms
     assert n1 == n2 and n1 > lines
+    for s, n in zip(picks, counts):
+        assert n == pytest.approx(_lines_crossings(w.mesh, s, 5 if w.useReflections else 1), rel=1e-3)
 
 
 @pytest.mark.parametrize("reflections", [False, True])
