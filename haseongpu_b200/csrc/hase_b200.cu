@@ -793,9 +793,10 @@ __device__ __forceinline__ uint32_t warpUpperBound(const uint32_t* a, uint32_t n
     return lo;
 }
 
-// log2 of the entries between warpEntries' offsets for `rays` rays in `entries` entries.
+// log2 of the entries between warpEntries' offsets for `rays` rays in `entries`
+// entries; at most 26, so that b0 + (32 << shift) stays below 2^32 for b0 < 2^31.
 __device__ __forceinline__ uint32_t entryShift(uint32_t entries, uint32_t rays) {
-    return entries <= rays ? 0u : 31u - uint32_t(__clz(int(2u * entries / rays)));
+    return entries <= rays ? 0u : min(26u, 31u - uint32_t(__clz(int(2u * (entries / rays)))));
 }
 
 // Start state of ray r of sample `sample`, drawn in reflection slice j and
