@@ -410,7 +410,6 @@ struct hase_proposal {
     hase::DevBuf<int> error;   // set by a kernel whose tensor-core wait timed out
     // training state
     hase::DevBuf<float> dparams, adamM, adamV, grad, loss;
-    hase::DevBuf<float> gradRows, groupLoss;  // a step's sums: one gradient row per CTA, one loss term per group
     hase::DevBuf<float> lossHistory;
-    hase::DevBuf<unsigned char> batchRows;  // the last call's rows (DeviceBatch)
+    hase::DevBuf<unsigned char> batchRows;  // the last call's rows and sums (DeviceBatch)
 };

@@ -657,13 +657,15 @@ hase_status hase_proposal_forward(hase_proposal* net, uint32_t rows, const float
 
 namespace {
 
-// A call's rows on the device, in one block of the network's (batchRows).
+// A call's rows and its steps' sums on the device, in one block of the
+// network's (batchRows).
 struct DeviceBatch {
     uint32_t groups = 0, rows = 0;
     std::vector<uint32_t> offsets;
     uint32_t* doffsets = nullptr;
     float *features = nullptr, *targets = nullptr, *logits = nullptr, *dl = nullptr;
     float* weights = nullptr;  // or null: every group weighs the same
+    float *gradRows = nullptr, *groupLoss = nullptr;  // StepSums
 };
 
 // The block stays with the network up to this size, so that the calls of a
@@ -699,7 +701,8 @@ hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, Device
         return at;
     };
     const size_t atOffsets = place(size_t(b->groups) + 1), atFeatures = place(rows * kFeat), atTargets = place(rows),
-                 atLogits = place(rows), atDl = place(rows), atWeights = place(b->groupWeights ? b->groups : 0);
+                 atLogits = place(rows), atDl = place(rows), atWeights = place(b->groupWeights ? b->groups : 0),
+                 atGrad = place(size_t(2u * net->numSMs) * kGradStride), atLoss = place(b->groups);
     HASE_CUDA(net->batchRows.ensure(bytes));
     unsigned char* const base = net->batchRows.p;
     d.doffsets = reinterpret_cast<uint32_t*>(base + atOffsets);
@@ -708,6 +711,8 @@ hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, Device
     d.logits = reinterpret_cast<float*>(base + atLogits);
     d.dl = reinterpret_cast<float*>(base + atDl);
     d.weights = b->groupWeights ? reinterpret_cast<float*>(base + atWeights) : nullptr;
+    d.gradRows = reinterpret_cast<float*>(base + atGrad);
+    d.groupLoss = reinterpret_cast<float*>(base + atLoss);
     const auto send = [&](void* to, const void* from, size_t n) {
         return cudaMemcpyAsync(to, from, n * 4, cudaMemcpyHostToDevice, net->stream);
     };
@@ -723,7 +728,7 @@ hase_status uploadBatch(hase_proposal* net, const hase_proposal_batch* b, Device
 hase_status lossGrad(hase_proposal* net, DeviceBatch& d, uint32_t g0, uint32_t g1, float* dLoss, StepSums& out) {
     const uint32_t r0 = d.offsets[g0], r1 = d.offsets[g1];
     const uint32_t rows = r1 - r0;
-    out = StepSums{net->gradRows.p, net->groupLoss.p, dLoss, 0u, 0u};
+    out = StepSums{d.gradRows, d.groupLoss, dLoss, 0u, 0u};
     if (rows == 0) return HASE_OK;
     const uint32_t tiles = (rows + kTile - 1) / kTile;
     const uint32_t grid = std::min(tiles, 2u * net->numSMs);  // two CTAs per SM
@@ -734,10 +739,10 @@ hase_status lossGrad(hase_proposal* net, DeviceBatch& d, uint32_t g0, uint32_t g
     mlpForwardKernel<<<fgrid, kTile, kSmemBytes, net->stream>>>(F);
     HASE_CUDA(cudaGetLastError());
     StatsLaunch S{d.logits, d.targets, d.weights, d.doffsets, g0, 0u,
-                  1.0f / float(g1 - g0), d.dl, net->groupLoss.p};
+                  1.0f / float(g1 - g0), d.dl, d.groupLoss};
     groupStatsKernel<<<g1 - g0, kStatsBlock, 0, net->stream>>>(S);
     HASE_CUDA(cudaGetLastError());
-    TrainLaunch T{net->wimg.p, net->vec.p, d.features + size_t(r0) * kFeat, d.dl + r0, rows, net->gradRows.p,
+    TrainLaunch T{net->wimg.p, net->vec.p, d.features + size_t(r0) * kFeat, d.dl + r0, rows, d.gradRows,
                   net->error.p};
     mlpBackwardKernel<<<grid, kTile, kTrainSmemBytes, net->stream>>>(T);
     HASE_CUDA(cudaGetLastError());
@@ -749,7 +754,6 @@ hase_status prepareTraining(hase_proposal* net) {
     HASE_CUDA(cudaFuncSetAttribute(mlpForwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)));
     HASE_CUDA(
         cudaFuncSetAttribute(mlpBackwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTrainSmemBytes)));
-    HASE_CUDA(net->gradRows.ensure(size_t(2u * net->numSMs) * kGradStride));
     return HASE_OK;
 }
 
@@ -765,7 +769,6 @@ hase_status hase_proposal_loss_grad(hase_proposal* net, const hase_proposal_batc
     HASE_TRY(uploadBatch(net, batch, d));
     HASE_CUDA(net->grad.ensure(HASE_PROPOSAL_PARAMS));
     HASE_CUDA(net->loss.ensure(1));
-    HASE_CUDA(net->groupLoss.ensure(d.groups));
     StepSums sums;
     HASE_TRY(lossGrad(net, d, 0, d.groups, net->loss.p, sums));
     gradientSumKernel<<<kSumBlocks, dim3(kSumParams, kSumLanes), 0, net->stream>>>(sums, net->grad.p);
@@ -792,7 +795,6 @@ hase_status hase_proposal_train(hase_proposal* net, const hase_proposal_batch* b
     const float eps = tr->epsilon > 0.0f ? tr->epsilon : 1e-8f;
     DevBuf<float>& hist = net->lossHistory;
     HASE_CUDA(hist.ensure(tr->steps));
-    HASE_CUDA(net->groupLoss.ensure(tr->groupsPerStep));
     HASE_CUDA(net->dparams.ensure(HASE_PROPOSAL_PARAMS));
     HASE_CUDA(net->adamM.ensure(HASE_PROPOSAL_PARAMS));
     HASE_CUDA(net->adamV.ensure(HASE_PROPOSAL_PARAMS));
