@@ -399,6 +399,11 @@ constexpr uint32_t kMaxGridY = 65535;  // blocks of a grid in y
 // rows).  A point's lines -- its requested levels x slices x layers -- fill the
 // narrowest team that holds them with at most 4 per lane, in as few chunks of
 // a full warp as there must be; the lines per lane then as even as they go.
+// 4 per lane take 117 registers (two blocks per SM) and 3 per lane 78 (three),
+// but a chunk walks the segment again: with at most 4 against at most 3 per
+// lane 16 lines 1.98 / 2.65 ms, 56 0.94 / 1.38, 110 1.91 / 2.69, 200 5.66 / 6.24,
+// 240 3.74 / 4.20, 290 5.53 / 5.57, 380 2.29 / 2.35; only 16 candidate triangles
+// with 290 lines, two blocks to a sample, prefer 3 (2.02 / 1.92).
 // count: the counting kernel (il.crossings accumulates the walk's crossings).
 cudaError_t launchImportance(ImportanceLaunch il, uint32_t meshLayers, uint32_t T, uint32_t Np, uint32_t rows,
                              cudaStream_t stream, bool count = false) {
@@ -1122,11 +1127,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) rayKernel(RayLaunch L) {
 // Launch shapes of rayKernel the autotuner chooses from: block size, idle
 // lanes that trigger a refill, the occupancy target (blocks per SM the
 // register budget is fitted to) and the triangle columns a lane walks per
-// step call (32 unless named).  Entry 0 is the default: 64 registers a thread
-// without spills beat five blocks of 48 with 50 to 110 bytes of them wherever
-// both were timed (5,470 mono samples 27.7 against 29.7 ms, 256 polychromatic
-// ones 4.66 / 4.86, 512 with grid weights 8.59 / 8.98, 5-sample query 21 us
-// both).  Single-medium shapes also carry the kernels of the other walk modes.
+// step call (32 unless named).  Entry 0 is the default: 64 registers a thread,
+// without spills (pooled 20 to 28 bytes), where five blocks of 48 registers
+// spill 40 to 96 (pooled 140 to 188).  It is the fastest shape, against the best
+// of 48 registers (256 threads, refill 16, 64 columns), with 256 polychromatic
+// samples (4.51 / 4.57 ms), 512 with grid weights (8.37 / 8.49), 1,024 cladded
+// ones (4.78 / 5.04), 128 mono ones (0.672 / 0.676) and 12 media in a batch (2.58 /
+// 2.69), and within 1 us of it on a 5-sample query (23 us).  On all 5,470 mono
+// samples the other one wins (25.8 / 25.4): a long monochromatic solve is what
+// the autotuner is for.  Single-medium shapes also carry the kernels of the
+// other walk modes.
 struct RayVariant {
     void (*kernel)(RayLaunch);
     int block;

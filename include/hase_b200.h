@@ -197,9 +197,10 @@ hase_status hase_grid_weights(hase_context* ctx, uint32_t firstSample, uint32_t 
 
 /* Crossings of the importance walks of samples [firstSample, firstSample +
  * count): per (sample, reflection slice, prism) line, the triangles its 2-D
- * projection crosses plus the level planes and reflections on the way -- the
- * work unit of the importance kernel's roofline (counted by an instrumented
- * copy of the kernel; the walks are those of hase_calc_phi_ase). */
+ * projection crosses plus the level planes and reflections on the way.  The
+ * count is of the lines; the kernel steps through the triangles and takes the
+ * planes between them from a table (an instrumented copy of the kernel; the
+ * lines are those of hase_calc_phi_ase). */
 hase_status hase_importance_crossings(hase_context* ctx, uint32_t firstSample, uint32_t count,
                                       uint32_t useReflections, uint64_t* crossings);
 
