@@ -45,8 +45,13 @@ sys.path.insert(0, str(REPO))
 
 METRIC = ("phi-ASE time to per-sample relative error <= threshold on 1 B200, as sample points solved per second "
           "(rays/s alongside)")
-FP32_INSTR_PER_CROSSING = 24   # stated per-crossing FP32 instruction count
+# stated per-crossing FP32 instruction count: two edges' exit parameters 7 each, the choice between them 3, the
+# segment's end 2, the level plane 2, the gain 2, the advance 1
+FP32_INSTR_PER_CROSSING = 24
 BYTES_PER_CROSSING = 36        # a triangle's window of two edges 32 B + prism value 4 B
+# FP32 and integer operations of an importance line in one triangle: position, table entry and its distance at the
+# exit 5, the comparison with the next bounce 1, the integral 4, two table addresses
+OPS_PER_LINE_STEP = 12
 SMS = 148
 LANES_PER_SM = 128
 MLP_FLOP_PER_PAIR = 2 * (12 * 64 + 64 * 64 + 64 * 64 + 64 * 1)  # 18,048 FLOP per (sample, prism) inference
@@ -58,15 +63,16 @@ XU_LANES_PER_SM = 16
 FWD_METRIC = "forward Tet4 phi-ASE source rays traced and tallied per second on 1 B200 (crossings/s alongside)"
 FP64_INSTR_PER_TET_CROSSING = 100  # stated per-crossing FP64 instruction count of the forward walk
 BYTES_PER_TET_CROSSING = 148       # cell record 128 B + beta 8 B + one vertex tally 8 B + one visit count 4 B
-FWD_TRAFFIC_DISC_POLY = 49128192   # DRAM bytes of one fwdRayKernel launch on the disc_poly Tet4 twin (ncu)
+FWD_TRAFFIC_DISC_POLY = 49300480   # DRAM bytes of one fwdRayKernel launch on the disc_poly Tet4 twin (ncu)
 FP64_LANES_PER_SM = 64
-# DRAM bytes of one learned-solve rayKernel launch on disc_small (5,470 samples x 1e5 rays; ncu): the per-sample
-# ray maps (q, offsets) read once and the per-item partial sums written; the walk tables stay in L1/L2
-RAY_TRAFFIC_LEARNED = 402847744 + 29695232
-# what binds the same launch (ncu --set full of it): instruction issue, with the walk tables in L1 -- thread
-# instructions per crossing and per ray of that capture (3.09e10 warp instructions x 24.4 threads, 5.47e8 rays)
-RAY_BINDING_LEARNED = "instruction issue (ncu: issue active 85.6 %, top stall 'not selected'; L1 hits 99.2 %)"
-RAY_INSTR_LEARNED = {"per_crossing": 97, "per_ray": 1379, "crossings_per_ray": 14.2}
+# ncu of a learned-solve rayKernel launch on disc_small's mesh with 1,024 samples x 1e5 rays (256 threads, 64 columns,
+# 512 rays per item): DRAM bytes, scaled to 5,470 samples (the per-sample ray maps read once and the per-item partial
+# sums written: both per sample), and what binds it -- instruction issue, with the walk tables in L1 -- with its thread
+# instructions per crossing and per ray (4.22e9 warp instructions x 27.2 threads, 1.02e8 rays)
+RAY_TRAFFIC_LEARNED = (75_370_240 + 5_234_432) * 5470 // 1024
+RAY_BINDING_LEARNED = ("instruction issue (ncu, 1,024 samples: issue active 82.1 %, top stall 'not selected'; L1 hits "
+                       "95.7 %)")
+RAY_INSTR_LEARNED = {"per_crossing": 89, "per_ray": 1123, "crossings_per_ray": 12.7}
 
 
 def parse():
@@ -107,6 +113,22 @@ def measured_peaks():
     if p.exists():
         return json.loads(p.read_text()), "measured"
     return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "sm_max_mhz": 1965.0}, "fallback"
+
+
+def level_planes(mesh, first, count, slices):
+    """Level planes that the straight lines of `count` samples from `first` cross: from every prism with a source to every
+    image of the sample point.  The importance kernel does not step through them (hase_importance_crossings counts them)."""
+    import numpy as np
+
+    layers = mesh.numberOfLevels - 1
+    source = (np.asarray(mesh.betaVolume).reshape(layers, -1) > 0).sum(axis=1).astype(float)
+    level, samples = np.unique(np.arange(first, first + count) // mesh.numberOfPoints, return_counts=True)
+    centre = np.arange(layers) + 0.5
+    total = 0.0
+    for ls, n in zip(level, samples):
+        for image in [ls, -ls, 2 * layers - ls, ls - 2 * layers, ls + 2 * layers][:slices]:
+            total += n * (source * np.floor(np.abs(centre - image))).sum()
+    return total
 
 
 def cpu_baseline(workload, seconds, fields=None, nearField=False):
@@ -320,8 +342,10 @@ def measure_importance(args, local, rank=0, world=1, nested=False):
     ctx.update_beta(mesh.betaVolume)
 
     # crossings of the timed steps' importance walks (an instrumented copy of the kernel, untimed)
-    imp_crossings = sum(ctx.importance_crossings(((args.warmup + s) * world + rank) * B % (S - B + 1), B,
-                                                 w.useReflections) for s in range(args.steps))
+    firsts = [((args.warmup + s) * world + rank) * B % (S - B + 1) for s in range(args.steps)]
+    imp_crossings = sum(ctx.importance_crossings(f, B, w.useReflections) for f in firsts)
+    # one line in one triangle: what the importance kernel does once, whatever the number of levels in between
+    line_steps = imp_crossings - sum(level_planes(mesh, f, B, 5 if w.useReflections else 1) for f in firsts)
     # the plain method (uniform start points, as the legacy code) on one batch, for comparison
     plain = ctx.calc_phi_ase(minRays=w.minRays, maxRays=w.maxRays, mseThreshold=w.threshold,
                              useReflections=w.useReflections, monochromatic=w.monochromatic,
@@ -418,16 +442,17 @@ def measure_importance(args, local, rank=0, world=1, nested=False):
                          "achieved": achieved, "peak": roof, "unit": "crossings/s", "frac": achieved / roof,
                          "traffic": None, "fp32_issue_peak": r_fp32, "l2_gather_peak": r_l2,
                          "l2_read_gbs_live": l2, "clock_mhz": f_clk / 1e6, "peak_source": peak_kind},
-            "importance_roofline": {"bound": "fp32_issue" if r_fp32 <= r_l2 else "l2_gather",
-                                    "kernel": "importanceTeamKernel",
-                                    "achieved": imp_crossings / (imp_ms * 1e-3), "peak": roof, "unit": "crossings/s",
-                                    "frac": imp_crossings / (imp_ms * 1e-3) / roof,
-                                    "fp32_issue_frac": imp_crossings / (imp_ms * 1e-3) / r_fp32,
-                                    "crossings_per_step": imp_crossings / args.steps,
+            "importance_roofline": {"bound": "fp32_issue", "kernel": "importanceTeamKernel",
+                                    "achieved": line_steps / (imp_ms * 1e-3),
+                                    "peak": SMS * LANES_PER_SM * f_clk / OPS_PER_LINE_STEP, "unit": "line steps/s",
+                                    "frac": line_steps / (imp_ms * 1e-3)
+                                    / (SMS * LANES_PER_SM * f_clk / OPS_PER_LINE_STEP),
+                                    "line_steps_per_step": line_steps / args.steps,
                                     "ms_per_step": imp_ms / args.steps,
-                                    "walks_per_step": B * mesh.numberOfPrisms * (5 if w.useReflections else 1),
-                                    "note": "crossings: per (sample, slice, prism) line, triangles crossed by its "
-                                            "2-D projection plus level planes and reflections (in-kernel counter)"},
+                                    "lines_per_step": B * mesh.numberOfPrisms * (5 if w.useReflections else 1),
+                                    "note": "line steps: per (sample, slice, prism) line, the triangles that its 2-D "
+                                            "projection crosses (in-kernel counter of the crossings less the level "
+                                            "planes, which the kernel does not step through)"},
             "clocks": clocks,
             "wall_s": wall,
         }
@@ -1197,7 +1222,7 @@ def run_learned(args):
                          "achieved": achieved, "peak": roof, "unit": "crossings/s", "frac": achieved / roof,
                          "traffic": RAY_TRAFFIC_LEARNED,
                          "traffic_note": "DRAM bytes per launch (ncu): the per-sample ray maps read once and the "
-                                         "per-item partial sums; the walk tables stay in L1 (99 % hits) and L2",
+                                         "per-item partial sums; the walk tables stay in L1 (96 % hits) and L2",
                          "fp32_issue_peak": r_fp32, "l2_gather_peak": r_l2, "l1_gather_peak": r_l1,
                          "fp32_issue_frac": achieved / r_fp32, "l1_gather_frac": achieved / r_l1,
                          "l2_read_gbs_live": l2, "l1_read_gbs_live": l1, "smem_read_gbs_live": smem,
