@@ -3627,7 +3627,7 @@ hase_status hase_log_contributions(hase_context* c, const hase_experiment_desc* 
     return calcCore(c, ex, cp, res ? res : &local, nullptr, contributions);
 }
 
-constexpr size_t kFeatureFloats = size_t(4) << 20;  // hase_proposal_features' block of rows
+constexpr size_t kKeptFeatureFloats = size_t(4) << 20;  // hase_proposal_features: rows kept on the device
 
 hase_status hase_proposal_features(hase_context* c, uint32_t firstSample, uint32_t count, uint32_t useReflections,
                                    uint32_t monochromatic, float* features) {
@@ -3646,26 +3646,22 @@ hase_status hase_proposal_features(hase_context* c, uint32_t firstSample, uint32
     }
     ProposalView pv{};
     HASE_TRY(buildProposalView(c, A, B, pv));
+    pv.firstSample = firstSample;
     pv.nW = nW;
     localFields(c, pv);
-    // in blocks of rows through a buffer that stays with the context (16 MB, or
-    // one row: that is given back): allocating and freeing one for the whole call
-    // took 0.8 of the 2.2 ms of 32 samples of 9,126 prisms
-    const size_t row = size_t(nW) * kFeat;
-    const uint32_t perBlock = uint32_t(std::max<size_t>(1, std::min<size_t>(count, kFeatureFloats / row)));
+    const size_t n = size_t(count) * nW * kFeat;
+    // rows of up to 16 MB go through a buffer that stays with the context
+    // (allocating and freeing one per call took 0.8 of the 2.2 ms of 32 samples of
+    // 9,126 prisms), more through one that the call gives back: their copy takes
+    // tens of ms (in blocks of 16 MB instead it took a tenth longer)
     DevBuf<float> own;
-    DevBuf<float>& out = row <= kFeatureFloats ? c->featRows : own;
-    HASE_CUDA(out.ensure(perBlock * row));
-    for (uint32_t at = 0; at < count; at += perBlock) {
-        const uint32_t rows = std::min(perBlock, count - at);
-        pv.firstSample = firstSample + at;
-        ProposalLaunch pl{pv, nullptr, nullptr, nullptr, nullptr, out.p, rows, nullptr};
-        const uint64_t pairs = uint64_t(rows) * nW;
-        featureKernel<<<uint32_t((pairs + 255) / 256), 256, 0, c->stream>>>(pl);
-        HASE_CUDA(cudaGetLastError());
-        HASE_CUDA(cudaMemcpyAsync(features + at * row, out.p, rows * row * sizeof(float), cudaMemcpyDeviceToHost,
-                                  c->stream));
-    }
+    DevBuf<float>& out = n <= kKeptFeatureFloats ? c->featRows : own;
+    HASE_CUDA(out.ensure(n));
+    ProposalLaunch pl{pv, nullptr, nullptr, nullptr, nullptr, out.p, count, nullptr};
+    const uint64_t pairs = uint64_t(count) * nW;
+    featureKernel<<<uint32_t((pairs + 255) / 256), 256, 0, c->stream>>>(pl);
+    HASE_CUDA(cudaGetLastError());
+    HASE_CUDA(cudaMemcpyAsync(features, out.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     HASE_CUDA(cudaStreamSynchronize(c->stream));
     return HASE_OK;
 }

@@ -218,9 +218,9 @@ def test_fallback_restarts_samples_with_the_importance_weights(small, trained):
     assert none.fallbackSamples == 0 and np.all(none.totalRays == 80000)
 
 
-def test_features_come_in_bounded_blocks(small):
-    """Rows of more than one 16 MB block (38 of 9,126 pairs or 7 of 45,630, the last block a ragged one) are the single
-    rows, and the context keeps no more than the block."""
+def test_features_leave_a_bounded_buffer(small):
+    """Rows of less and more than 16 MB (38 of 9,126 pairs or 7 of 45,630) are the single rows, and the context keeps no
+    more than 16 MB of them."""
     import torch
 
     from haseongpu_b200 import DeviceMesh
