@@ -90,13 +90,18 @@ struct TetView {
 __device__ __forceinline__ double unit53(uint32_t x) { return (double(x >> 8) + 0.5) * (1.0 / 16777216.0); }
 
 // 256-bit read-only loads (sm_100): one 32-byte sector per lane and instruction.
-// They allocate no L1 lines: a large mesh's records are not met again before
-// they are evicted (5 % hits), and the lines they took cost the reductions and
-// the beta reads theirs (287,622 cells, 4M rays: 7.66 -> 6.99 ms; 17,496 cells:
-// no difference).
+// STREAM: they allocate no L1 lines.  A large mesh's records are not met again
+// before they are evicted (5 % hits), and the lines they took cost the
+// reductions and the beta reads theirs; a small mesh's are (kStreamCells).
+template <bool STREAM>
 __device__ __forceinline__ double4 ldPlane(const double4* p) {
     double4 v;
-    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    if (STREAM)
+        asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+            : "l"(p));
+    else
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
     return v;
 }
 
@@ -105,12 +110,19 @@ struct CellLinks {
     uint4 matv;
 };
 
+template <bool STREAM = true>
 __device__ __forceinline__ CellLinks ldLinks(const int4* p) {
     CellLinks l;
-    asm("ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(l.nbr.x), "=r"(l.nbr.y), "=r"(l.nbr.z), "=r"(l.nbr.w), "=r"(l.matv.x), "=r"(l.matv.y),
-          "=r"(l.matv.z), "=r"(l.matv.w)
-        : "l"(p));
+    if (STREAM)
+        asm("ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(l.nbr.x), "=r"(l.nbr.y), "=r"(l.nbr.z), "=r"(l.nbr.w), "=r"(l.matv.x), "=r"(l.matv.y),
+              "=r"(l.matv.z), "=r"(l.matv.w)
+            : "l"(p));
+    else
+        asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(l.nbr.x), "=r"(l.nbr.y), "=r"(l.nbr.z), "=r"(l.nbr.w), "=r"(l.matv.x), "=r"(l.matv.y),
+              "=r"(l.matv.z), "=r"(l.matv.w)
+            : "l"(p));
     return l;
 }
 
@@ -118,13 +130,14 @@ __device__ __forceinline__ CellLinks ldLinks(const int4* p) {
 // along u, the entry face ff excluded: among the faces with dlambda < 0, the
 // smallest max(lambda, 0) / -dlambda (lowest index on a tie).  Fills lam and
 // dl for all four faces; returns -1 when no face decreases.
+template <bool STREAM>
 __device__ __forceinline__ int exitFace(const double4* __restrict__ pl, double x, double y, double z, double ux,
                                         double uy, double uz, int ff, double lam[4], double dl[4], double& len) {
     int bf = -1;
     double bl = 0.0, bd = -1.0;
 #pragma unroll
     for (int f = 1; f < 4; ++f) {
-        const double4 p = ldPlane(pl + f - 1);
+        const double4 p = ldPlane<STREAM>(pl + f - 1);
         lam[f] = fma(p.x, x, fma(p.y, y, fma(p.z, z, p.w)));
         dl[f] = fma(p.x, ux, fma(p.y, uy, p.z * uz));
     }
@@ -439,8 +452,8 @@ namespace {
 // MODE 0: source rays; 1: source rays that deposit at reflecting faces (the
 // first pass of the surface-reservoir method); 2: reflected rays drawn from
 // the reservoir, depositing in turn (blocks of a batch whose chain has ended
-// return at once).
-template <bool SMEM, int MODE>
+// return at once).  STREAM: how the cell records are read (ldPlane).
+template <bool SMEM, int MODE, bool STREAM>
 __global__ void __launch_bounds__(kFwdBlock, kFwdMinBlocks) fwdRayKernel(const FwdLaunch L) {
     extern __shared__ double hist[];
     const TetView& m = L.m;
@@ -493,7 +506,7 @@ __global__ void __launch_bounds__(kFwdBlock, kFwdMinBlocks) fwdRayKernel(const F
 #pragma unroll 1
         for (int k = 0; k < kFwdSteps && live; ++k) {
             double lam[4], dl[4], len;
-            const int bf = exitFace(m.cell[r.c].plane, r.x, r.y, r.z, r.ux, r.uy, r.uz, r.ff, lam, dl, len);
+            const int bf = exitFace<STREAM>(m.cell[r.c].plane, r.x, r.y, r.z, r.ux, r.uy, r.uz, r.ff, lam, dl, len);
             bool drop = bf < 0 || ++r.steps > kFwdMaxSteps;
             const int n = bf == 0 ? r.nbr.x : bf == 1 ? r.nbr.y : bf == 2 ? r.nbr.z : r.nbr.w;
             if (!drop) {
@@ -516,7 +529,7 @@ __global__ void __launch_bounds__(kFwdBlock, kFwdMinBlocks) fwdRayKernel(const F
             } else {
                 r.c = uint32_t(n) >> 2;
                 r.ff = n & 3;
-                const CellLinks lk = ldLinks(&m.cell[r.c].nbr);
+                const CellLinks lk = ldLinks<STREAM>(&m.cell[r.c].nbr);
                 r.nbr = lk.nbr;
                 carryPending(r, bf, r.ff, lk.matv, m.Np, add);
             }
@@ -530,6 +543,19 @@ __global__ void __launch_bounds__(kFwdBlock, kFwdMinBlocks) fwdRayKernel(const F
         }
     }
 }
+
+using FwdKernel = void (*)(const FwdLaunch);
+template <bool STREAM>
+FwdKernel fwdKernel(bool smem, int mode) {
+    if (smem) return mode == 0 ? fwdRayKernel<true, 0, STREAM> : mode == 1 ? fwdRayKernel<true, 1, STREAM> : fwdRayKernel<true, 2, STREAM>;
+    return mode == 0 ? fwdRayKernel<false, 0, STREAM> : mode == 1 ? fwdRayKernel<false, 1, STREAM> : fwdRayKernel<false, 2, STREAM>;
+}
+
+// Cells (128 bytes each) above which the records are read without allocating L1
+// lines.  Allocating against not, 3M rays: 162 cells 5.75 / 5.96 ms, 576 5.21 / 5.37,
+// 5,760 3.33 / 3.44, 12,600 3.15 / 3.22 (300,000 rays 0.35 / 0.33), 21,294 3.63 / 3.54,
+// 196,794 5.14 / 4.72; 287,622 cells, 4M rays 7.66 / 6.99.
+constexpr uint32_t kStreamCells = 12000;
 
 struct FinLaunch {
     const double* score;   // [B][2 Np]
@@ -798,7 +824,7 @@ __global__ void __launch_bounds__(128) fwdTraceKernel(const TraceLaunch T) {
     while (seg < uint32_t(kFwdMaxSteps)) {
         double lam[4], dl[4], len;
         const TetCell* rec = m.cell + r.c;
-        const int bf = exitFace(rec->plane, r.x, r.y, r.z, r.ux, r.uy, r.uz, r.ff, lam, dl, len);
+        const int bf = exitFace<true>(rec->plane, r.x, r.y, r.z, r.ux, r.uy, r.uz, r.ff, lam, dl, len);
         if (bf < 0) break;
         lg += gainCoefficient(m, r.c, T.sA, T.sE) * len;
         if (seg < T.maxSegments) {
@@ -1336,18 +1362,14 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
     if (smem && histBytes > kMaxHistogramBytes)
         return fail(HASE_INVALID_ARGUMENT, "shared-memory tallies need 2 * numberOfPoints * 8 <= %zu bytes",
                     kMaxHistogramBytes);
+    const auto kernel = [&](int mode) {
+        return C > kStreamCells ? fwdKernel<true>(smem, mode) : fwdKernel<false>(smem, mode);
+    };
     int perSM = 0;
-    if (smem) {
-        HASE_CUDA(cudaFuncSetAttribute(fwdRayKernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(histBytes)));
-        HASE_CUDA(cudaFuncSetAttribute(fwdRayKernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(histBytes)));
-        HASE_CUDA(cudaFuncSetAttribute(fwdRayKernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(histBytes)));
-        HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fwdRayKernel<true, 0>, block, histBytes));
-    } else {
-        HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fwdRayKernel<false, 0>, block, 0));
-    }
+    if (smem)
+        for (int mode = 0; mode < 3; ++mode)
+            HASE_CUDA(cudaFuncSetAttribute(kernel(mode), cudaFuncAttributeMaxDynamicSharedMemorySize, int(histBytes)));
+    HASE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel(0), block, smem ? histBytes : 0));
     // surface-reservoir controls (include/core/types.hpp:328-330, src/core/srm.cpp:36-41)
     const uint32_t srmMaxIt = fw->reflectionMaxIterations ? fw->reflectionMaxIterations : 40u;
     const double srmTol = fw->reflectionTolerance > 0.0 ? fw->reflectionTolerance : 1.0e-4;
@@ -1489,8 +1511,7 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
             const uint32_t grid = perBatch * B;
             const size_t shm = smem ? histBytes : 0;
             if (!srm || nF == 0) {
-                if (smem) fwdRayKernel<true, 0><<<grid, block, shm, c->stream>>>(L);
-                else fwdRayKernel<false, 0><<<grid, block, shm, c->stream>>>(L);
+                kernel(0)<<<grid, block, shm, c->stream>>>(L);
                 HASE_CUDA(cudaGetLastError());
                 res->kernelLaunches += 1;
             } else {
@@ -1534,11 +1555,9 @@ extern "C" hase_status hase_tet_calc_phi_ase(hase_tet_context* c, const hase_for
                             const Philox4 o = philox4x32_10(b, launch, pass, kTagFwdBatch, fw->rngSeed, kFwdKeyHi);
                             L.shift[b] = double(o.x) / 4294967296.0;
                         }
-                        if (smem) fwdRayKernel<true, 2><<<grid, block, shm, c->stream>>>(L);
-                        else fwdRayKernel<false, 2><<<grid, block, shm, c->stream>>>(L);
+                        kernel(2)<<<grid, block, shm, c->stream>>>(L);
                     } else {
-                        if (smem) fwdRayKernel<true, 1><<<grid, block, shm, c->stream>>>(L);
-                        else fwdRayKernel<false, 1><<<grid, block, shm, c->stream>>>(L);
+                        kernel(1)<<<grid, block, shm, c->stream>>>(L);
                     }
                     HASE_CUDA(cudaGetLastError());
                     srmSortKernel<<<uint32_t((faces + 255) / 256), 256, 0, c->stream>>>(

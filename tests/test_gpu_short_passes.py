@@ -111,3 +111,29 @@ def test_group_statistics_at_block_edges(sizes):
             lse = np.log(np.exp(l - l.max()).sum()) + l.max()
             ref += (lse - (y * l).sum() / y.sum()) / len(sizes)
     assert loss == pytest.approx(ref, rel=1e-5, abs=1e-5)
+
+
+@pytest.mark.parametrize("rings,levels,streamed", [(3, 2, False), (9, 9, False), (9, 10, True)])
+@pytest.mark.parametrize("tally", ["global", "shared"])
+def test_cell_records_read_either_way(oracle, rings, levels, streamed, tally):
+    """Meshes below and above the 12,000 cells from which the records are read without allocating L1 lines start and walk
+    the oracle's rays: visits equal, phi to a few float ulps (the replay level)."""
+    from haseongpu_b200 import PrismMesh, TetDeviceMesh, TetMesh
+    from haseongpu_b200.mesh import delaunay_triangles, disc_points
+
+    rng = np.random.default_rng(rings)
+    pts = disc_points(1.0, rings, rng)
+    tri = delaunay_triangles(pts)
+    T = tri.shape[0]
+    mesh = TetMesh.fromPrismMesh(PrismMesh(points=pts, triangles=tri, numberOfLevels=levels, thickness=0.7 / (levels - 1),
+                                           betaVolume=rng.uniform(0.05, 0.3, T * (levels - 1)), nTot=1e20,
+                                           crystalTFluo=1e-3))
+    assert (mesh.numberOfCells > 12_000) == streamed
+    spectrum = ([1e-21], [2e-20])
+    ref = oracle.forward_phi_ase(mesh, spectrum, minRays=20_000, seed=3)
+    with TetDeviceMesh(mesh, *spectrum) as ctx:
+        dev = ctx.calc_phi_ase(forwardRayCount=20_000, rngSeed=3, tallyMode=tally)
+    assert (dev.totalRays != ref["rayVisits"]).mean() < 2e-3
+    live = ref["phiAse"] > 0
+    rel = np.abs(dev.phiAse[live] / ref["phiAse"][live] - 1.0)
+    assert np.quantile(rel, 0.999) < 1e-5
